@@ -7,10 +7,6 @@
 
 namespace hx {
 
-Engine::~Engine() {
-  if (dev_args_) cudaFree(dev_args_);
-}
-
 // Host-side check of every launch shape against the window layout (planner.h); a violation is
 // a bug in the planner, reported instead of launched.
 #define HX_CHECK_PLAN(KIND, G, AMOUNT)                                                   \
@@ -24,26 +20,6 @@ Engine::~Engine() {
 
 LaunchShape Engine::shape(const Geometry& g) const {
   return LaunchShape{g.ctas, g.threads, world() ? int(views.size()) : 0};
-}
-
-// Production: the single argument block is passed by value. World: the blocks of all ranks go
-// to device memory first (stream-ordered copy from the caller's vector, which outlives it
-// because the copy of pageable memory returns only after the source was read).
-template <typename Args>
-const Args* Engine::stage(const std::vector<Args>& args, cudaStream_t st, cudaError_t* rc) {
-  *rc = cudaSuccess;
-  if (!world()) return args.data();
-  const size_t bytes = args.size() * sizeof(Args);
-  if (bytes > dev_args_bytes_) {
-    if (dev_args_) cudaFree(dev_args_);
-    dev_args_ = nullptr;
-    if ((*rc = cudaMalloc(&dev_args_, bytes)) != cudaSuccess) return nullptr;
-    dev_args_bytes_ = bytes;
-  }
-  // earlier launches may still read the buffer
-  if ((*rc = cudaStreamSynchronize(st)) != cudaSuccess) return nullptr;
-  *rc = cudaMemcpyAsync(dev_args_, args.data(), bytes, cudaMemcpyHostToDevice, st);
-  return static_cast<const Args*>(dev_args_);
 }
 
 cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpPlan& plan,
@@ -79,7 +55,6 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
     }
   }
   last_variant = var;
-  cudaError_t rc;
   ++launches;
   if (var == kVarLL) {
     const size_t lines = (bytes + 7) / 8;
@@ -91,8 +66,7 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
       build_allreduce_ll(&args[r], views[r], epoch, b[r].send, b[r].recv, count, dt, plan, order,
                          tune.nvls && tune.ll_mc && !world());
     epoch += 1;
-    const LLArgs* a = stage(args, st, &rc);
-    return rc != cudaSuccess ? rc : launch_ll(dt, a, shape(g), st);
+    return launch_ll(dt, args.data(), shape(g), st);
   }
   if (var == kVarOneShot) {
     // the recursive-doubling order costs n log n combines per element: give a CTA less of it
@@ -103,8 +77,7 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
     for (size_t r = 0; r < views.size(); ++r)
       build_allreduce_oneshot(&args[r], views[r], epoch, g, b[r].send, b[r].recv, count, dt, plan, order);
     epoch += g.epochs;
-    const XchgArgs* a = stage(args, st, &rc);
-    return rc != cudaSuccess ? rc : launch_xchg_fold(dt, a, shape(g), st);
+    return launch_xchg_fold(dt, args.data(), shape(g), st);
   }
   if (var == kVarRing) {
     const size_t es = dtype_size(dt);
@@ -114,8 +87,7 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
     for (size_t r = 0; r < views.size(); ++r)
       build_allreduce_twoshot(&args[r], views[r], epoch, g, b[r].send, b[r].recv, count, dt, plan, order, false);
     epoch += g.epochs;
-    const TwoShotArgs* a = stage(args, st, &rc);
-    return rc != cudaSuccess ? rc : launch_ring(dt, a, shape(g), st);
+    return launch_ring(dt, args.data(), shape(g), st);
   }
   // The three-role pipeline wins for the multicast reduction from three ranks on; for the
   // exact two-shot it measured faster than the single-role kernel only on eight ranks.
@@ -140,10 +112,8 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
     build_allreduce_twoshot(&args[r], views[r], epoch, g, b[r].send, b[r].recv, count, dt, plan,
                             order, tune.nvls && tune.nvls_gather && roles && n() > 2 && bytes % 16 == 0);
   epoch += g.epochs;
-  const TwoShotArgs* a = stage(args, st, &rc);
-  if (rc != cudaSuccess) return rc;
   if (roles) last_variant = kVarTwoShotRoles;
-  return roles ? launch_twoshot_roles(dt, a, shape(g), st) : launch_twoshot(dt, a, shape(g), st);
+  return roles ? launch_twoshot_roles(dt, args.data(), shape(g), st) : launch_twoshot(dt, args.data(), shape(g), st);
 }
 
 cudaError_t Engine::allreduce_cast(const RankBufs* b, size_t count, int wire_dt, const OpPlan& plan,
@@ -157,9 +127,7 @@ cudaError_t Engine::allreduce_cast(const RankBufs* b, size_t count, int wire_dt,
   epoch += g.epochs;
   ++launches;
   last_variant = kVarTwoShot;
-  cudaError_t rc;
-  const TwoShotArgs* a = stage(args, st, &rc);
-  return rc != cudaSuccess ? rc : launch_twoshot_cast(wire_dt, a, shape(g), st);
+  return launch_twoshot_cast(wire_dt, args.data(), shape(g), st);
 }
 
 cudaError_t Engine::reducescatter(const RankBufs* b, size_t per, int dt, const OpPlan& plan,
@@ -179,9 +147,7 @@ cudaError_t Engine::reducescatter(const RankBufs* b, size_t per, int dt, const O
       build_reducescatter_ring(&args[r], views[r], epoch, g, b[r].send, b[r].recv, per, dt, plan);
     epoch += g.epochs;
     ++launches;
-    cudaError_t rc;
-    const TwoShotArgs* a = stage(args, st, &rc);
-    return rc != cudaSuccess ? rc : launch_ring(dt, a, shape(g), st);
+    return launch_ring(dt, args.data(), shape(g), st);
   }
   const Geometry g = plan_xchg(per * dtype_size(dt), n(), views[0].half_bytes, tune);
   HX_CHECK_PLAN(kPlanXchg, g, per * dtype_size(dt));
@@ -190,9 +156,7 @@ cudaError_t Engine::reducescatter(const RankBufs* b, size_t per, int dt, const O
     build_reducescatter(&args[r], views[r], epoch, g, b[r].send, b[r].recv, per, dt, plan);
   epoch += g.epochs;
   ++launches;
-  cudaError_t rc;
-  const XchgArgs* a = stage(args, st, &rc);
-  return rc != cudaSuccess ? rc : launch_xchg_fold(dt, a, shape(g), st);
+  return launch_xchg_fold(dt, args.data(), shape(g), st);
 }
 
 cudaError_t Engine::reduce(const RankBufs* b, size_t count, int dt, const OpPlan& plan, int root,
@@ -204,9 +168,7 @@ cudaError_t Engine::reduce(const RankBufs* b, size_t count, int dt, const OpPlan
     build_reduce(&args[r], views[r], epoch, g, b[r].send, b[r].recv, count, dt, plan, root);
   epoch += g.epochs;
   ++launches;
-  cudaError_t rc;
-  const XchgArgs* a = stage(args, st, &rc);
-  return rc != cudaSuccess ? rc : launch_xchg_fold(dt, a, shape(g), st);
+  return launch_xchg_fold(dt, args.data(), shape(g), st);
 }
 
 #define HX_COPY_COLLECTIVE(MAXPAIR, BUILD)                                  \
@@ -216,9 +178,7 @@ cudaError_t Engine::reduce(const RankBufs* b, size_t count, int dt, const OpPlan
   for (size_t r = 0; r < views.size(); ++r) { BUILD; }                      \
   epoch += g.epochs;                                                         \
   ++launches;                                                               \
-  cudaError_t rc;                                                           \
-  const XchgArgs* a = stage(args, st, &rc);                                 \
-  return rc != cudaSuccess ? rc : launch_xchg_copy(a, shape(g), st);
+  return launch_xchg_copy(args.data(), shape(g), st);
 
 cudaError_t Engine::allgather(const RankBufs* b, size_t block, cudaStream_t st) {
   // AllGather moves the same bytes into every rank whichever way they are pushed, so multicast
@@ -302,7 +262,16 @@ cudaError_t Engine::p2p(const RankP2p* ops, cudaStream_t st) {
     error = "Send/Recv lanes of " + std::to_string(n()) + " ranks cannot be co-resident on this device";
     return cudaErrorInvalidValue;
   }
-  for (;;) {  // a lane takes kMaxLaneOps operations per launch; more go into another round
+  // A lane takes kMaxLaneOps operations per launch; more go into another round. A world's launch
+  // carries the lanes of all ranks in one parameter, so a very full group takes more rounds of
+  // fewer operations per lane (the same number on every lane: both ends of a lane stay paired).
+  int lane_ops = kMaxLaneOps;
+  if (world()) {
+    size_t total = 0;
+    for (size_t r = 0; r < nr; ++r) total += left[r].size();
+    while (lane_ops > 1 && total > size_t(kWorldMaxOps) && nr * size_t(most_lanes) * size_t(lane_ops) > size_t(kWorldMaxOps)) lane_ops /= 2;
+  }
+  for (;;) {
     bool any = false;
     std::vector<P2pArgs> args(nr);
     int max_lanes = 0;
@@ -328,7 +297,7 @@ cudaError_t Engine::p2p(const RankP2p* ops, cudaStream_t st) {
         const bool blocked = std::any_of(rest.begin(), rest.end(), [&](const P2pOp& q) {
           return q.peer == o.peer && q.is_send == o.is_send;
         });
-        if (lane < 0 || blocked || a.lanes[lane].nops == kMaxLaneOps) {
+        if (lane < 0 || blocked || a.lanes[lane].nops == lane_ops) {
           rest.push_back(o);
           continue;
         }
@@ -342,10 +311,7 @@ cudaError_t Engine::p2p(const RankP2p* ops, cudaStream_t st) {
     }
     if (!any) return cudaSuccess;
     ++launches;
-    cudaError_t rc;
-    const P2pArgs* a = stage(args, st, &rc);
-    if (rc != cudaSuccess) return rc;
-    rc = launch_p2p(a, LaunchShape{max_lanes * (kP2pWorkers / wpc), threads, world() ? int(nr) : 0}, st);
+    const cudaError_t rc = launch_p2p(args.data(), LaunchShape{max_lanes * (kP2pWorkers / wpc), threads, world() ? int(nr) : 0}, st);
     if (rc != cudaSuccess) return rc;
   }
 }

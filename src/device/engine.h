@@ -39,7 +39,6 @@ class Engine {
   unsigned long long launches = 0;  // kernels launched so far
   std::string error;
 
-  ~Engine();
   bool world() const { return views.size() > 1; }
   int n() const { return views[0].n; }
 
@@ -62,12 +61,8 @@ class Engine {
   cudaError_t p2p(const RankP2p* ops, cudaStream_t st);
 
  private:
-  template <typename Args>
-  const Args* stage(const std::vector<Args>& args, cudaStream_t st, cudaError_t* rc);
   LaunchShape shape(const Geometry& g) const;
   uint64_t ll_era_ = 0;  // upper half of the epoch the line region was last cleared for
-  void* dev_args_ = nullptr;
-  size_t dev_args_bytes_ = 0;
 };
 
 }  // namespace hx

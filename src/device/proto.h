@@ -208,5 +208,20 @@ struct P2pArgs {
   int bulk;                  // senders move their pieces with bulk asynchronous copies (needs the dynamic shared memory)
   P2pLane lanes[kMaxLanes];  // CTA (lane, group) = blockIdx.x / G, % G with G = kP2pWorkers / workers_per_cta
 };
+// The lanes of every rank of a single-GPU world, packed (16 full P2pArgs would not fit the 32 KB
+// of a launch's parameters).
+struct P2pWorldLane {
+  uint16_t first_op;
+  uint8_t nops, peer, is_send;
+};
+constexpr int kWorldMaxOps = 1024, kWorldMaxLanes = kMaxRanks * 2 * (kMaxRanks - 1);
+template <int kLanes, int kOps>
+struct P2pWorldArgs {
+  WinView w[kMaxRanks];
+  int workers_per_cta;
+  uint16_t lane0[kMaxRanks + 1];  // rank r's lanes are [lane0[r], lane0[r + 1])
+  P2pWorldLane lane[kLanes];
+  P2pLaneOp ops[kOps];
+};
 
 }  // namespace hx

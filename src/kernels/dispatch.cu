@@ -13,19 +13,23 @@ __global__ void __launch_bounds__(512) k_xchg_copy(const __grid_constant__ XchgA
   __shared__ FoldShared sh;
   xchg_body<uint8_t, false>(a, blockIdx.x, gridDim.x, sh);
 }
-__global__ void __launch_bounds__(512) k_xchg_copy_world(const XchgArgs* a) {
+__global__ void __launch_bounds__(512) k_xchg_copy_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
   __shared__ FoldShared sh;
-  xchg_body<uint8_t, false>(a[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  xchg_body<uint8_t, false>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 // CTA (lane, group): the group's workers one after the other (see P2pArgs::workers_per_cta)
-__device__ inline void p2p_cta(const P2pArgs& a, int* fail, unsigned long long* word, BulkPipe* pipe = nullptr) {
-  const int wpc = a.workers_per_cta, groups = kP2pWorkers / wpc;
-  const int lane = blockIdx.x / groups, first = (blockIdx.x % groups) * wpc;
-  if (lane >= a.nlanes) return;
+__device__ inline void p2p_workers(const WinView& w, const P2pLaneView& lane, int group, int wpc, int* fail,
+                                   unsigned long long* word, BulkPipe* pipe = nullptr) {
   for (int k = 0; k < wpc; ++k) {
-    if (!p2p_body(a, lane, first + k, fail, word, pipe)) return;
+    if (!p2p_body(w, lane, group * wpc + k, fail, word, pipe)) return;
     __syncthreads();
   }
+}
+__device__ inline void p2p_cta(const P2pArgs& a, int* fail, unsigned long long* word, BulkPipe* pipe = nullptr) {
+  const int groups = kP2pWorkers / a.workers_per_cta, lane = blockIdx.x / groups;
+  if (lane >= a.nlanes) return;
+  const P2pLane& l = a.lanes[lane];
+  p2p_workers(a.w, P2pLaneView{l.peer, l.is_send, l.nops, l.ops}, blockIdx.x % groups, a.workers_per_cta, fail, word, pipe);
 }
 __global__ void __launch_bounds__(512) k_p2p(const __grid_constant__ P2pArgs a) {
   __shared__ int fail;
@@ -43,10 +47,16 @@ __global__ void __launch_bounds__(512) k_p2p_bulk(const __grid_constant__ P2pArg
   bulk_pipe_init(pipe, staging, bars);
   p2p_cta(a, &fail, &word, &pipe);
 }
-__global__ void __launch_bounds__(512) k_p2p_world(const P2pArgs* a) {
+template <int kLanes, int kOps>
+__global__ void __launch_bounds__(512) k_p2p_world(const __grid_constant__ P2pWorldArgs<kLanes, kOps> a) {
   __shared__ int fail;
   __shared__ unsigned long long word;
-  p2p_cta(a[blockIdx.y], &fail, &word);
+  const int groups = kP2pWorkers / a.workers_per_cta, r = blockIdx.y;
+  const int lane = a.lane0[r] + blockIdx.x / groups;
+  if (lane >= a.lane0[r + 1]) return;
+  const P2pWorldLane& l = a.lane[lane];
+  p2p_workers(a.w[r], P2pLaneView{l.peer, l.is_send, l.nops, a.ops + l.first_op}, blockIdx.x % groups, a.workers_per_cta,
+              &fail, &word);
 }
 template <typename T, int kMode>
 __global__ void __launch_bounds__(512) k_nvls(const __grid_constant__ NvlsArgs a) {
@@ -117,8 +127,38 @@ cudaError_t launch_xchg_copy(const XchgArgs* args, LaunchShape s, cudaStream_t s
   return cudaGetLastError();
 }
 
+template <int kLanes, int kOps>
+static cudaError_t launch_p2p_world(const P2pArgs* args, LaunchShape s, cudaStream_t st) {
+  P2pWorldArgs<kLanes, kOps> a;
+  static_assert(sizeof a <= 32764, "kernel parameters");
+  if (s.world > kMaxRanks) return cudaErrorInvalidValue;
+  int lane = 0, op = 0;
+  a.workers_per_cta = args[0].workers_per_cta;
+  for (int r = 0; r < s.world; ++r) {
+    a.w[r] = args[r].w;
+    a.lane0[r] = uint16_t(lane);
+    for (int k = 0; k < args[r].nlanes; ++k) {
+      const P2pLane& l = args[r].lanes[k];
+      a.lane[lane++] = P2pWorldLane{uint16_t(op), uint8_t(l.nops), uint8_t(l.peer), uint8_t(l.is_send)};
+      for (int q = 0; q < l.nops; ++q) a.ops[op++] = l.ops[q];
+    }
+  }
+  a.lane0[s.world] = uint16_t(lane);
+  void* params[] = {&a};
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(&k_p2p_world<kLanes, kOps>), dim3(s.ctas, s.world), dim3(s.threads),
+                                     params, 0, st);
+}
 cudaError_t launch_p2p(const P2pArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world) return launch_world(reinterpret_cast<const void*>(&k_p2p_world), args, s, st);
+  if (s.world) {
+    size_t lanes = 0, ops = 0;
+    for (int r = 0; r < s.world; ++r) {
+      lanes += size_t(args[r].nlanes);
+      for (int k = 0; k < args[r].nlanes; ++k) ops += size_t(args[r].lanes[k].nops);
+    }
+    if (lanes <= 128 && ops <= 128) return launch_p2p_world<128, 128>(args, s, st);  // a quarter of the parameter bytes
+    if (lanes <= size_t(kWorldMaxLanes) && ops <= size_t(kWorldMaxOps)) return launch_p2p_world<kWorldMaxLanes, kWorldMaxOps>(args, s, st);
+    return cudaErrorInvalidValue;
+  }
   if (args->bulk) {
     static const cudaError_t opted = cudaFuncSetAttribute(k_p2p_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBulkSmemBytes));
     if (opted != cudaSuccess) return opted;

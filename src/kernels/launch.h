@@ -1,8 +1,8 @@
 // Host-callable launchers of the sm_100a kernels. `world` > 1 launches the single-GPU
-// "whole world in one grid" form: args then points to `world` argument blocks in device
-// memory and blockIdx.y selects the rank (cooperative launch, so all ranks' CTAs are
-// co-resident and can wait on one another). world == 0 launches the production form with
-// the one argument block passed by value.
+// "whole world in one grid" form: args then points to `world` argument blocks and blockIdx.y
+// selects the rank (cooperative launch, so all ranks' CTAs are co-resident and can wait on one
+// another). world == 0 launches the production form with one argument block. The blocks are host
+// memory and travel as kernel parameters either way.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -20,9 +20,7 @@ using namespace hx;
 constexpr size_t kHalf = 512 * 1024;
 constexpr size_t kWindow = 256 * 1024 + 2 * kHalf;
 static_assert(kOffFlagsB + size_t(kMaxCtas) * kMaxRanks * 8 <= 256 * 1024, "flag pages must fit the header");
-constexpr size_t kArgsOff = HXCCL_NOALLOC_MAX_RANKS * kWindow;
-constexpr size_t kStatusOff = kArgsOff + 8192;  // 2 words per rank
-static_assert(HXCCL_NOALLOC_MAX_RANKS * sizeof(XchgArgs) <= 8192, "argument blocks must fit");
+constexpr size_t kStatusOff = HXCCL_NOALLOC_MAX_RANKS * kWindow;  // 2 words per rank
 constexpr size_t kScratchBytes = kStatusOff + 256;
 
 // The scratch. In host code this name is only a handle for cudaGetSymbolAddress: it is not a
@@ -130,12 +128,7 @@ extern "C" hxcclResult_t hxcclAllReduceNoAlloc(int nranks, const void* const* se
     build_allreduce_oneshot(&args[r], w, pd.epoch, g, send[r], recv[r], count, dt, plan, order);
   }
   pd.epoch += g.epochs;
-  const XchgArgs* dev_args = reinterpret_cast<const XchgArgs*>(pd.base + kArgsOff);
-  e = cudaMemcpyAsync(pd.base + kArgsOff, args, sizeof(XchgArgs) * nranks, cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return fail(hxcclUnhandledCudaError, "staging the arguments", e);
-  // `args` lives on this stack frame: the copy of pageable memory has read it by now, and the
-  // function does not return before the stream is idle anyway
-  e = launch_xchg_fold(dt, dev_args, LaunchShape{g.ctas, g.threads, nranks}, st);
+  e = launch_xchg_fold(dt, args, LaunchShape{g.ctas, g.threads, nranks}, st);
   if (e != cudaSuccess) {
     pd.dirty = true;
     return fail(hxcclUnhandledCudaError, "launching the AllReduce kernel", e);

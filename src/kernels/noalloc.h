@@ -4,10 +4,9 @@
 // where cudaMalloc is off limits: inside a region whose memory is owned by a caching allocator
 // that forbids raw allocations, in a process that has pinned its whole device-memory budget up
 // front, or in late start-up / teardown paths where the allocator is not (or no longer) usable.
-// Such callers can still check the collective kernels on one GPU: the staging windows, the
-// per-rank argument blocks and the status words all live in one file-scope device array of
-// fixed size that is part of the library image, so the call allocates nothing, neither on the
-// device nor in pinned host memory.
+// Such callers can still check the collective kernels on one GPU: the staging windows and the
+// status words live in one file-scope device array of fixed size that is part of the library
+// image, so the call allocates nothing, neither on the device nor in pinned host memory.
 #pragma once
 #include <stddef.h>
 
@@ -32,12 +31,12 @@ extern "C" {
  * size beyond the maximum; last error text via hxcclNoAllocLastError), hxcclTimeout when a
  * device-side wait ran out, hxcclUnhandledCudaError for CUDA failures.
  *
- * Scratch: one static device array of 5 251 328 bytes (5.0 MiB) per GPU that loads the
+ * Scratch: one static device array of 5 243 136 bytes (5.0 MiB) per GPU that loads the
  * library, held until the process exits. The first call on a device is the set-up: with that
  * device current it looks the array's device address up (cudaGetSymbolAddress) and clears the
  * array; make that first call before any stream capture begins. Later calls repeat the look-up
- * (so a device reset cannot leave a stale pointer behind). Every call copies its argument
- * blocks from pageable host memory and ends with cudaStreamSynchronize(stream).
+ * (so a device reset cannot leave a stale pointer behind). Every call ends with
+ * cudaStreamSynchronize(stream).
  * Every call uses the same array and finds what the previous call left there: flags only grow
  * from call to call and the status words are cleared at the start of each call. Two calls that
  * overlap on the GPU (different streams, or different threads) therefore race on the array;

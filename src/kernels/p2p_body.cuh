@@ -50,10 +50,12 @@ __device__ __forceinline__ unsigned long long p2p_rounds(size_t total, size_t sl
 }
 
 // One worker's share of every operation of a lane. False when a wait gave up.
-__device__ inline bool p2p_body(const P2pArgs& a, int lane_idx, int wk, int* sh_fail, unsigned long long* sh_word,
+struct P2pLaneView {
+  int peer, is_send, nops;
+  const P2pLaneOp* ops;
+};
+__device__ inline bool p2p_body(const WinView& w, const P2pLaneView& lane, int wk, int* sh_fail, unsigned long long* sh_word,
                                 BulkPipe* pipe = nullptr) {
-  const WinView& w = a.w;
-  const P2pLane& lane = a.lanes[lane_idx];
   const int me = w.rank, peer = lane.peer;
   char* mine = w.win[me];
   char* theirs = w.win[peer];
