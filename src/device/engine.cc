@@ -25,10 +25,16 @@ LaunchShape Engine::shape(const Geometry& g) const {
 cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpPlan& plan,
                               int order, cudaStream_t st) {
   const size_t bytes = count * dtype_size(dt);
-  // One rank, nothing to scale or divide: the result is the input (the reference's path does a
-  // plain copy then too, src/algo_ring.cc:17-18). In place that is no work at all.
-  if (!world() && n() == 1 && !plan.premul && !(plan.postdiv && plan.divisor != 1)) {
+  // One rank: the result is the input (the reference's path does a plain copy then too,
+  // src/algo_ring.cc:17-18; in place that is no work at all), or the input times the scalar.
+  if (!world() && n() == 1 && !(plan.postdiv && plan.divisor != 1)) {
     last_variant = kVarAuto;
+    if (plan.premul) {
+      ++launches;
+      unsigned long long bits = 0;
+      std::memcpy(&bits, plan.scalar, 8);
+      return launch_scale(b[0].recv, b[0].send, count, dt, bits, plan.scalar_dev, st);
+    }
     if (b[0].send == b[0].recv) return cudaSuccess;
     ++launches;
     return launch_copy(b[0].recv, b[0].send, bytes, st);

@@ -23,7 +23,8 @@ __device__ __forceinline__ size_t min_sz(size_t a, size_t b) { return a < b ? a 
 // AllGather, AlltoAll(v), Broadcast, Gather, Scatter (copy mode); ReduceScatter, Reduce and the
 // one-shot AllReduce (fold mode) are all "push blocks into peers' windows, hand over, take
 // what arrived".
-template <typename T, bool kFold>
+// kN: see cta_fold (fold mode).
+template <typename T, bool kFold, int kN = 0>
 __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) {
   const WinView& w = a.w;
   const int me = w.rank, n = w.n;
@@ -48,16 +49,16 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
     size_t by_mc = 0;  // bytes of this step's piece that went out through the switch's multicast
     if (!kFold && a.mc_bytes > lo)
       by_mc = cta_copy_multicast(w.mc + slot_off, a.mc_src + lo, min_sz(a.sub_bytes, a.mc_bytes - lo));
-    for (int jj = 1; jj < n; ++jj) {
-      const int j = (me + jj) % n;
-      if (a.send_bytes[j] <= lo + by_mc) continue;
-      const size_t len = min_sz(a.sub_bytes, a.send_bytes[j] - lo) - by_mc;
-      char* to = w.win[j] + slot_off + by_mc;
-      if (kFold && a.push_scaled)
-        cta_scale_copy<T>(to, a.send_ptr[j] + lo, len, scalar);
-      else
-        cta_copy(to, a.send_ptr[j] + lo + by_mc, len);
+    if (threadIdx.x + 1 < unsigned(n)) {  // piece jj - 1 goes to rank me + jj
+      const int j = (me + 1 + int(threadIdx.x)) % n;
+      sh.piece_src[threadIdx.x] = a.send_ptr[j] + lo + by_mc;
+      sh.piece_dst[threadIdx.x] = w.win[j] + slot_off + by_mc;
+      sh.piece_len[threadIdx.x] = a.send_bytes[j] > lo + by_mc ? min_sz(a.sub_bytes, a.send_bytes[j] - lo) - by_mc : 0;
     }
+    if (kFold && a.push_scaled)
+      cta_pieces(sh, n - 1, a.sub_bytes, ScaleMover<T>{scalar});
+    else
+      cta_pieces(sh, n - 1, a.sub_bytes, CopyMover{});
     __syncthreads();
     tm.lap(kTrIn);
     signal_all(w, kOffFlagsA, cta, e_step0 + step);
@@ -67,13 +68,15 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
     const size_t lo = (size_t(step) * ncta + cta) * a.sub_bytes;
     const size_t buf = stg.at(step);
     if (!kFold) {
-      for (int ii = 0; ii < n; ++ii) {
-        const int i = (me + ii) % n;
-        if (a.recv_bytes[i] <= lo) continue;
-        const size_t len = min_sz(a.sub_bytes, a.recv_bytes[i] - lo);
+      if (threadIdx.x < unsigned(n)) {
+        const int i = (me + int(threadIdx.x)) % n;
         const char* from = i == me ? a.send_ptr[me] + lo : mine + buf + size_t(i) * a.slot_stride + in_slot;
-        if (from != a.recv_ptr[i] + lo) cta_copy(a.recv_ptr[i] + lo, from, len);
+        char* to = a.recv_ptr[i] + lo;
+        sh.piece_src[threadIdx.x] = from;
+        sh.piece_dst[threadIdx.x] = to;
+        sh.piece_len[threadIdx.x] = a.recv_bytes[i] > lo && from != to ? min_sz(a.sub_bytes, a.recv_bytes[i] - lo) : 0;
       }
+      cta_pieces(sh, n, a.sub_bytes, CopyMover{});
     } else if (a.fold_bytes > lo) {
       const size_t len = min_sz(a.sub_bytes, a.fold_bytes - lo);
       __syncthreads();  // the previous fold is done with sh.src
@@ -83,35 +86,30 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
       }
       if (threadIdx.x == 0) sh.mc_dst = nullptr;
       __syncthreads();
-      cta_fold<T>(a.fold_dst + lo, sh, 0, len, a.fold_elem0 + lo / sizeof(T), a.fold, me, n, scalar);
+      cta_fold<T, kN>(a.fold_dst + lo, sh, 0, len, a.fold_elem0 + lo / sizeof(T), a.fold, a.fold.premul != 0, me, n, scalar);
     }
   };
 
-  if (!multi) {
-    push(0);
-    if (!wait_all(w, kOffFlagsA, cta, e_step0, &sh.fail)) return;
-    tm.lap(kTrWaitA);
-    consume(0);
-    __syncthreads();
-    tm.lap(kTrOut);
-    tm.done();
-    return;
+  if (multi) {  // entry
+    if (!signal_and_wait(w, kOffFlagsA, cta, a.epoch0, &sh.fail)) return;
+    tm.lap(kTrWaitB);
   }
-  if (!signal_and_wait(w, kOffFlagsA, cta, a.epoch0, &sh.fail)) return;  // entry
-  tm.lap(kTrWaitB);
-  push(0);
-  for (int k = 0; k < a.steps; ++k) {
+  // one push and one consume in the text: each is inlined once
+  for (int k = -1; k < a.steps; ++k) {
     // push(k+1) reuses the buffer of step k-3. The owner consumed that step before it pushed
     // step k-1, and this CTA saw the owner's signal of step k-1 in the previous iteration.
     if (k + 1 < a.steps) push(k + 1);
+    if (k < 0) continue;
     if (!wait_all(w, kOffFlagsA, cta, e_step0 + k, &sh.fail)) return;
     tm.lap(kTrWaitA);
     consume(k);
     __syncthreads();
     tm.lap(kTrOut);
   }
-  signal_and_wait(w, kOffFlagsA, cta, e_step0 + a.steps, &sh.fail);  // closing
-  tm.lap(kTrWaitB);
+  if (multi) {
+    signal_and_wait(w, kOffFlagsA, cta, e_step0 + a.steps, &sh.fail);  // closing
+    tm.lap(kTrWaitB);
+  }
   tm.done();
 }
 
@@ -130,7 +128,7 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
 // reads n sources of T as always; the fold leaves the own slice's result in the window, and the
 // gather widens every slice, the own one included, into the fp32 output. Bit for bit this is
 // "cast to T, AllReduce in T, cast back".
-template <typename T, bool kCast = false>
+template <typename T, int kN, bool kCast = false>
 __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared& sh) {
   const WinView& w = a.w;
   const int me = w.rank, n = w.n;
@@ -153,19 +151,21 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
   // fold instead of stalling the CTA twice per step.
   auto push = [&](int step, bool signal) {  // phase A: my contribution to every other owner's slice
     const size_t step0 = size_t(step) * n * slice, buf = stg.at(step);
-    for (int jj = kCast ? 0 : 1; jj < n; ++jj) {
-      const int j = (me + jj) % n;
+    const int np = kCast ? n : n - 1;
+    if (threadIdx.x < unsigned(np)) {
+      const int j = (me + (kCast ? 0 : 1) + int(threadIdx.x)) % n;
       const size_t lo = step0 + size_t(j) * slice + in_slice;
-      if (lo >= a.bytes) continue;
-      const size_t len = min_sz(a.sub_bytes, a.bytes - lo);
-      char* to = w.win[j] + buf + size_t(me) * slice + in_slice;
-      if constexpr (kCast)
-        cta_narrow_scale_copy<T>(to, reinterpret_cast<const float*>(a.send) + lo / sizeof(T), len, scalar,
-                                 a.fold.premul != 0);
-      else if (a.fold.premul)
-        cta_scale_copy<T>(to, a.send + lo, len, scalar);
+      sh.piece_src[threadIdx.x] = a.send + (kCast ? lo / sizeof(T) * sizeof(float) : lo);
+      sh.piece_dst[threadIdx.x] = w.win[j] + buf + size_t(me) * slice + in_slice;
+      sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
+    }
+    if constexpr (kCast) {
+      cta_pieces(sh, np, a.sub_bytes, NarrowMover<T>{scalar, a.fold.premul != 0});
+    } else {
+      if (a.fold.premul)
+        cta_pieces(sh, np, a.sub_bytes, ScaleMover<T>{scalar});
       else
-        cta_copy(to, a.send + lo, len);
+        cta_pieces(sh, np, a.sub_bytes, CopyMover{});
     }
     __syncthreads();
     tm.lap(kTrIn);
@@ -187,17 +187,9 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
     if (threadIdx.x == 0)
       sh.mc_dst = a.use_mc ? w.mc + buf + ag_base + size_t(me) * slice + in_slice : nullptr;
     __syncthreads();
-    if (lo < a.bytes) {
-      if (kCast) {  // every source is staged and already scaled; the result stays in the window
-        FoldSpec plain = a.fold;
-        plain.premul = 0;
-        cta_fold<T>(mine + buf + ag_base + size_t(me) * slice + in_slice, sh, n - 1,
-                    min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), plain, me, n, scalar);
-      } else {
-        cta_fold<T>(a.recv + lo, sh, n - 1, min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold,
-                    me, n, scalar);
-      }
-    }
+    if (lo < a.bytes)  // kCast: every source is staged and already scaled; the result stays in the window
+      cta_fold<T, kN>(kCast ? mine + buf + ag_base + size_t(me) * slice + in_slice : a.recv + lo, sh, n - 1,
+                  min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold, !kCast && a.fold.premul != 0, me, n, scalar);
     __syncthreads();
     tm.lap(kTrMid);
     signal_all(w, kOffFlagsB, cta, e_step0 + step);
@@ -206,53 +198,46 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
   };
   auto gather = [&](int step) {  // phase B: the other owners' results
     const size_t step0 = size_t(step) * n * slice, buf = stg.at(step);
-    for (int ii = kCast ? 0 : 1; ii < n; ++ii) {
-      const int i = (me + ii) % n;
+    const int np = kCast ? n : n - 1;
+    if (threadIdx.x < unsigned(np)) {
+      const int i = (me + (kCast ? 0 : 1) + int(threadIdx.x)) % n;
       const size_t lo = step0 + size_t(i) * slice + in_slice;
-      if (lo >= a.bytes) continue;
-      const char* from = mine + buf + ag_base + size_t(i) * slice + in_slice;
-      if constexpr (kCast)
-        cta_widen_copy<T>(reinterpret_cast<float*>(a.recv) + lo / sizeof(T), from, min_sz(a.sub_bytes, a.bytes - lo));
-      else
-        cta_copy(a.recv + lo, from, min_sz(a.sub_bytes, a.bytes - lo));
+      sh.piece_src[threadIdx.x] = mine + buf + ag_base + size_t(i) * slice + in_slice;
+      sh.piece_dst[threadIdx.x] = a.recv + (kCast ? lo / sizeof(T) * sizeof(float) : lo);
+      sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
+    if constexpr (kCast)
+      cta_pieces(sh, np, a.sub_bytes, WidenMover<T>{});
+    else
+      cta_pieces(sh, np, a.sub_bytes, CopyMover{});
     __syncthreads();
     tm.lap(kTrOut);
   };
 
-  if (!multi) {
-    push(0, true);
-    if (!wait_all(w, kOffFlagsA, cta, e_step0, &sh.fail)) return;
-    tm.lap(kTrWaitA);
-    fold(0, false);
-    if (!wait_all(w, kOffFlagsB, cta, e_step0, &sh.fail)) return;
-    tm.lap(kTrWaitB);
-    gather(0);
-    tm.done();
-    return;
-  }
-  if (!signal_and_wait(w, kOffFlagsA, cta, a.epoch0, &sh.fail)) return;  // entry
-  push(0, true);
-  for (int k = 0; k < a.steps; ++k) {
+  if (multi && !signal_and_wait(w, kOffFlagsA, cta, a.epoch0, &sh.fail)) return;  // entry
+  // one push, one fold and one gather in the text: each is inlined once
+  for (int k = -1; k <= a.steps; ++k) {
     // push(k+1) overwrites phase A slots of step k-3: their owners folded that step before
     // they signalled B(k-3), which this CTA waited for two iterations ago.
-    if (k + 1 < a.steps) push(k + 1, false);
-    if (!wait_all(w, kOffFlagsA, cta, e_step0 + k, &sh.fail)) return;
-    tm.lap(kTrWaitA);
-    // fold(k) overwrites phase B slots of step k-4 on the peers: a peer copied those out
-    // before it pushed step k-1 (signal A(k-1)), which is older than the A(k) just seen.
-    fold(k, k + 1 < a.steps);
+    if (k + 1 < a.steps) push(k + 1, k < 0);
+    if (k < 0) continue;
+    if (k < a.steps) {
+      if (!wait_all(w, kOffFlagsA, cta, e_step0 + k, &sh.fail)) return;
+      tm.lap(kTrWaitA);
+      // fold(k) overwrites phase B slots of step k-4 on the peers: a peer copied those out
+      // before it pushed step k-1 (signal A(k-1)), which is older than the A(k) just seen.
+      fold(k, k + 1 < a.steps);
+    }
     if (k > 0) {
       if (!wait_all(w, kOffFlagsB, cta, e_step0 + k - 1, &sh.fail)) return;
       tm.lap(kTrWaitB);
       gather(k - 1);
     }
   }
-  if (!wait_all(w, kOffFlagsB, cta, e_step0 + a.steps - 1, &sh.fail)) return;
-  tm.lap(kTrWaitB);
-  gather(a.steps - 1);
-  signal_and_wait(w, kOffFlagsA, cta, e_step0 + a.steps, &sh.fail);  // closing
-  tm.lap(kTrWaitB);
+  if (multi) {
+    signal_and_wait(w, kOffFlagsA, cta, e_step0 + a.steps, &sh.fail);  // closing
+    tm.lap(kTrWaitB);
+  }
   tm.done();
 }
 

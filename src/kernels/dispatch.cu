@@ -177,7 +177,7 @@ cudaError_t launch_p2p(const P2pArgs* args, LaunchShape s, cudaStream_t st) {
   extern template cudaError_t launch_ll_t<T>(const LLArgs*, LaunchShape, cudaStream_t);         \
   extern template cudaError_t launch_reduce_t<T>(void*, const void*, size_t, int, cudaStream_t); \
   extern template cudaError_t launch_scale_t<T>(void*, const void*, size_t, unsigned long long, \
-                                                cudaStream_t);                                  \
+                                                const void*, cudaStream_t);                     \
   extern template cudaError_t launch_divide_t<T>(void*, size_t, int, cudaStream_t);
 HX_EXTERN_TYPE(int8_t)
 HX_EXTERN_TYPE(uint8_t)
@@ -229,13 +229,17 @@ cudaError_t launch_reduce(void* dst, const void* src, size_t count, int dt, int 
   HX_DISPATCH_DTYPE(dt, rc = launch_reduce_t<T>(dst, src, count, op, st))
   return rc;
 }
+cudaError_t launch_scale(void* dst, const void* src, size_t count, int dt, unsigned long long scalar_bits,
+                         const void* scalar_dev, cudaStream_t st) {
+  cudaError_t rc = cudaErrorInvalidValue;
+  HX_DISPATCH_DTYPE(dt, rc = launch_scale_t<T>(dst, src, count, scalar_bits, scalar_dev, st))
+  return rc;
+}
 cudaError_t launch_scale(void* dst, const void* src, size_t count, int dt, const void* scalar_host,
                          cudaStream_t st) {
   unsigned long long bits = 0;
   memcpy(&bits, scalar_host, dtype_size(dt));
-  cudaError_t rc = cudaErrorInvalidValue;
-  HX_DISPATCH_DTYPE(dt, rc = launch_scale_t<T>(dst, src, count, bits, st))
-  return rc;
+  return launch_scale(dst, src, count, dt, bits, nullptr, st);
 }
 cudaError_t launch_divide(void* buf, size_t count, int dt, int divisor, cudaStream_t st) {
   cudaError_t rc = cudaErrorInvalidValue;

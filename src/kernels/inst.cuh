@@ -18,48 +18,49 @@ struct WorldArgs {
   Args rank[kMaxRanks];
 };
 
-template <typename T>
+// kN: the rank count the fold is unrolled for (see cta_fold, fold.cuh); HX_BY_RANKS picks it.
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_xchg_fold(const __grid_constant__ XchgArgs a) {
   __shared__ FoldShared sh;
-  xchg_body<T, true>(a, blockIdx.x, gridDim.x, sh);
+  xchg_body<T, true, kN>(a, blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_xchg_fold_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
   __shared__ FoldShared sh;
-  xchg_body<T, true>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  xchg_body<T, true, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot(const __grid_constant__ TwoShotArgs a) {
   __shared__ FoldShared sh;
-  twoshot_body<T>(a, blockIdx.x, gridDim.x, sh);
+  twoshot_body<T, kN>(a, blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
   __shared__ FoldShared sh;
-  twoshot_body<T>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  twoshot_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
 // fp32 buffers, T on the wire (instantiated for fp16 and bf16 only)
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot_cast(const __grid_constant__ TwoShotArgs a) {
   __shared__ FoldShared sh;
-  twoshot_body<T, true>(a, blockIdx.x, gridDim.x, sh);
+  twoshot_body<T, kN, true>(a, blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot_cast_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
   __shared__ FoldShared sh;
-  twoshot_body<T, true>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  twoshot_body<T, kN, true>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot_roles(const __grid_constant__ TwoShotArgs a) {
   __shared__ FoldShared sh;
-  twoshot_roles_body<T>(a, blockIdx.x, gridDim.x, sh);
+  twoshot_roles_body<T, kN>(a, blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(512) k_twoshot_roles_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
   __shared__ FoldShared sh;
-  twoshot_roles_body<T>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  twoshot_roles_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
 template <typename T>
@@ -94,35 +95,33 @@ cudaError_t launch_world(const void* kernel, const Args* args, LaunchShape s, cu
   return cudaLaunchCooperativeKernel(kernel, dim3(s.ctas, s.world), dim3(s.threads), params, 0, st);
 }
 
+// Launches KERNEL<T, kN>, or KERNEL_world<T, kN> for a world, for the rank count of args[0].
+#define HX_LAUNCH_RANKS(KERNEL, KN)                                                                       \
+  if (s.world) return launch_world(reinterpret_cast<const void*>(&KERNEL##_world<T, KN>), args, s, st);   \
+  KERNEL<T, KN><<<s.ctas, s.threads, 0, st>>>(*args);                                                     \
+  return cudaGetLastError()
+#define HX_BY_RANKS(KERNEL)                                                          \
+  const int n = args[0].w.n;                                                         \
+  if (n == 2) { HX_LAUNCH_RANKS(KERNEL, 2); }                                        \
+  if (n == 3 || n == 4) { HX_LAUNCH_RANKS(KERNEL, 4); }                              \
+  if (n > 4 && n <= kFastRanks) { HX_LAUNCH_RANKS(KERNEL, 8); }                      \
+  HX_LAUNCH_RANKS(KERNEL, 0)
+
 template <typename T>
 cudaError_t launch_xchg_fold_t(const XchgArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world)
-    return launch_world(reinterpret_cast<const void*>(&k_xchg_fold_world<T>), args, s, st);
-  k_xchg_fold<T><<<s.ctas, s.threads, 0, st>>>(*args);
-  return cudaGetLastError();
+  HX_BY_RANKS(k_xchg_fold);
 }
 template <typename T>
 cudaError_t launch_twoshot_t(const TwoShotArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world)
-    return launch_world(reinterpret_cast<const void*>(&k_twoshot_world<T>), args, s, st);
-  k_twoshot<T><<<s.ctas, s.threads, 0, st>>>(*args);
-  return cudaGetLastError();
+  HX_BY_RANKS(k_twoshot);
 }
-
 template <typename T>
 cudaError_t launch_twoshot_cast_t(const TwoShotArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world)
-    return launch_world(reinterpret_cast<const void*>(&k_twoshot_cast_world<T>), args, s, st);
-  k_twoshot_cast<T><<<s.ctas, s.threads, 0, st>>>(*args);
-  return cudaGetLastError();
+  HX_BY_RANKS(k_twoshot_cast);
 }
-
 template <typename T>
 cudaError_t launch_twoshot_roles_t(const TwoShotArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world)
-    return launch_world(reinterpret_cast<const void*>(&k_twoshot_roles_world<T>), args, s, st);
-  k_twoshot_roles<T><<<s.ctas, s.threads, 0, st>>>(*args);
-  return cudaGetLastError();
+  HX_BY_RANKS(k_twoshot_roles);
 }
 
 template <typename T>
@@ -150,22 +149,32 @@ __global__ void k_reduce(T* dst, const T* src, size_t n, int op) {
     Vec16<T> a, b;
     a.raw = ld16(reinterpret_cast<const char*>(dst) + (v << 4));
     b.raw = ld16(reinterpret_cast<const char*>(src) + (v << 4));
-    st16(reinterpret_cast<char*>(dst) + (v << 4), apply_lanes(a, b, op).raw);
+    st16(reinterpret_cast<char*>(dst) + (v << 4), combine_lanes(a, b, op).raw);
   }
   for (size_t e = nvec * V + tid; e < n; e += nth) dst[e] = apply(dst[e], src[e], op);
 }
+// dst = src * scalar; also the whole of an AllReduce over one rank that scales (Avg of floats,
+// PreMulSum). Bound by memory: warps take runs of four times 512 bytes, so that a thread has four loads
+// in flight. 28 MB fp32 in place (it stays in L2): 8.9 us; as a one-rank two-shot launch, whose
+// fold goes element by element for one rank and which ends in a hand-shake, 61.6 us.
 template <typename T>
-__global__ void k_scale(T* dst, const T* src, size_t n, unsigned long long scalar_bits) {
+__global__ void __launch_bounds__(256) k_scale(T* dst, const T* src, size_t n, unsigned long long scalar_bits,
+                                               const void* scalar_ptr) {
   T k;
-  memcpy(&k, &scalar_bits, sizeof(T));
-  constexpr int V = 16 / sizeof(T);
+  if (scalar_ptr) k = *static_cast<const T*>(scalar_ptr);
+  else memcpy(&k, &scalar_bits, sizeof(T));
+  constexpr int V = 16 / sizeof(T), U = 4;
   const size_t tid = blockIdx.x * size_t(blockDim.x) + threadIdx.x, nth = size_t(gridDim.x) * blockDim.x;
   const bool aligned = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
   const size_t nvec = aligned ? n / V : 0;
-  for (size_t v = tid; v < nvec; v += nth) {
-    Vec16<T> a;
-    a.raw = ld16(reinterpret_cast<const char*>(src) + (v << 4));
-    st16(reinterpret_cast<char*>(dst) + (v << 4), apply_lanes(a, splat(k), kProd).raw);
+  for (size_t v = (tid >> 5) * (32 * U) + (tid & 31u); v < nvec; v += nth * U) {
+    const char* from = reinterpret_cast<const char*>(src) + (v << 4);
+    char* to = reinterpret_cast<char*>(dst) + (v << 4);
+    Vec16<T> a[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) a[u].raw = ld16_if(v + u * 32 < nvec, from + u * 512);
+#pragma unroll
+    for (int u = 0; u < U; ++u) st16_if(v + u * 32 < nvec, to + u * 512, scale_lanes(a[u], k).raw);
   }
   for (size_t e = nvec * V + tid; e < n; e += nth) dst[e] = scale(src[e], k);
 }
@@ -189,9 +198,9 @@ cudaError_t launch_reduce_t(void* dst, const void* src, size_t count, int op, cu
 }
 template <typename T>
 cudaError_t launch_scale_t(void* dst, const void* src, size_t count, unsigned long long bits,
-                           cudaStream_t st) {
-  k_scale<T><<<elementwise_grid(count, 16 / sizeof(T)), 256, 0, st>>>(
-      static_cast<T*>(dst), static_cast<const T*>(src), count, bits);
+                           const void* scalar_ptr, cudaStream_t st) {
+  k_scale<T><<<elementwise_grid(count, 4 * 16 / sizeof(T)), 256, 0, st>>>(
+      static_cast<T*>(dst), static_cast<const T*>(src), count, bits, scalar_ptr);
   return cudaGetLastError();
 }
 template <typename T>
@@ -208,7 +217,7 @@ cudaError_t launch_divide_t(void* buf, size_t count, int divisor, cudaStream_t s
   template cudaError_t launch_ll_t<T>(const LLArgs*, LaunchShape, cudaStream_t);             \
   template cudaError_t launch_reduce_t<T>(void*, const void*, size_t, int, cudaStream_t);    \
   template cudaError_t launch_scale_t<T>(void*, const void*, size_t, unsigned long long,     \
-                                         cudaStream_t);                                      \
+                                         const void*, cudaStream_t);                         \
   template cudaError_t launch_divide_t<T>(void*, size_t, int, cudaStream_t);
 
 }  // namespace hx

@@ -38,6 +38,9 @@ cudaError_t launch_copy(void* dst, const void* src, size_t bytes, cudaStream_t s
 cudaError_t launch_reduce(void* dst, const void* src, size_t count, int dt, int op, cudaStream_t st);
 cudaError_t launch_scale(void* dst, const void* src, size_t count, int dt, const void* scalar_host,
                          cudaStream_t st);
+// the same with the scalar's bits (low bytes), or, where scalar_dev is not null, a device address to read it from
+cudaError_t launch_scale(void* dst, const void* src, size_t count, int dt, unsigned long long scalar_bits,
+                         const void* scalar_dev, cudaStream_t st);
 cudaError_t launch_divide(void* buf, size_t count, int dt, int divisor, cudaStream_t st);
 
 // largest grid of `threads`-wide CTAs of the widest collective kernel that is co-resident

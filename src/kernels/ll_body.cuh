@@ -61,8 +61,9 @@ __device__ inline bool ll_wait_line(const WinView& w, const char* line, unsigned
   }
 }
 
+// data[q]: the line of rank (me ^ q)
 template <typename T, int N>
-__device__ __forceinline__ T ll_fold_pow2(const uint2* data, int lane, int rank, int op) {
+__device__ __forceinline__ T ll_fold_pow2(const uint2* data, int lane, int op) {
   T x[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -71,7 +72,7 @@ __device__ __forceinline__ T ll_fold_pow2(const uint2* data, int lane, int rank,
     memcpy(e, &bits, 8);
     x[i] = e[lane];
   }
-  return fold_doubling_pow2<T, N>(x, rank, op);
+  return fold_doubling_pow2<T, N>(x, op);
 }
 
 // kN: the rank count when it is 2, 4 or 8 (loops unroll, every line lives in registers), else
@@ -125,23 +126,25 @@ __device__ void ll_ranks(const LLArgs& a, int cta, int ncta, FoldShared& sh) {
     }
   }
   // The lines of all sources are loaded together (their latencies overlap) and only those that
-  // have not arrived yet are polled one by one.
+  // have not arrived yet are polled one by one. With 2, 4 or 8 ranks the sources are taken as
+  // me ^ 0, me ^ 1, ..., the order in which recursive doubling is a plain tree (fold.cuh).
+  auto source = [&](int q) { return kFixed ? (me ^ q) : q; };
   for (size_t i = first; i < nlines; i += stride) {
     uint2 data[kN];
     uint4 seen[kN];
     const char* mine = w.win[me] + half + (i << 4);
 #pragma unroll
-    for (int p = 0; p < kN; ++p)
-      if (p < n && p != me) seen[p] = ld16_volatile(mine + size_t(p) * slot);
+    for (int q = 0; q < kN; ++q)
+      if (source(q) < n && source(q) != me) seen[q] = ld16_volatile(mine + size_t(source(q)) * slot);
     const uint2 own = own_line(i);
 #pragma unroll
-    for (int p = 0; p < kN; ++p) {
-      if (p >= n) continue;
-      if (p == me)
-        data[p] = own;
-      else if (seen[p].y == flag && seen[p].w == flag)
-        data[p] = make_uint2(seen[p].x, seen[p].z);
-      else if (!ll_wait_line(w, mine + size_t(p) * slot, flag, p, &data[p]))
+    for (int q = 0; q < kN; ++q) {
+      if (source(q) >= n) continue;
+      if (source(q) == me)
+        data[q] = own;
+      else if (seen[q].y == flag && seen[q].w == flag)
+        data[q] = make_uint2(seen[q].x, seen[q].z);
+      else if (!ll_wait_line(w, mine + size_t(source(q)) * slot, flag, source(q), &data[q]))
         return;
     }
 #pragma unroll
@@ -149,16 +152,16 @@ __device__ void ll_ranks(const LLArgs& a, int cta, int ncta, FoldShared& sh) {
       if (i * E + l >= total) break;
       T r;
       if (kFixed && f.kind == kFoldDoubling) {
-        r = ll_fold_pow2<T, kFixed ? kN : 2>(data, l, me, f.op);
+        r = ll_fold_pow2<T, kFixed ? kN : 2>(data, l, f.op);
       } else {
         T x[kN];
 #pragma unroll
-        for (int p = 0; p < kN; ++p) {
-          if (p >= n) continue;
-          const unsigned long long bits = (static_cast<unsigned long long>(data[p].y) << 32) | data[p].x;
+        for (int q = 0; q < kN; ++q) {
+          if (source(q) >= n) continue;
+          const unsigned long long bits = (static_cast<unsigned long long>(data[q].y) << 32) | data[q].x;
           T e[E];
           memcpy(e, &bits, 8);
-          x[p] = e[l];
+          x[source(q)] = e[l];
         }
         const int b = (f.kind == kFoldLinear && f.ring) ? ring_block_of(sh, i * E + l, n) : 0;
         r = fold_one(x, n, me, f, b);

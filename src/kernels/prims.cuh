@@ -1,6 +1,7 @@
 // Device-side building blocks: system-scope flag accesses, bounded waits, vector copies.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 #include "device/proto.h"
 #include "math/elem.h"
@@ -140,6 +141,25 @@ struct PhaseTimer {
 
 __device__ __forceinline__ uint4 ld16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ void st16(void* p, uint4 v) { *reinterpret_cast<uint4*>(p) = v; }
+// The same under a predicate, as one instruction each: written as `if (ok) r = ld16(p)`, unrolled
+// loads of a partial round become a ladder of branches that waits for one load before the next.
+// A load that does not take place gives zeros: left undefined, its registers would count as live
+// from the kernel's start, and every such loop would spill those of the others.
+__device__ __forceinline__ uint4 ld16_if(bool ok, const void* p) {
+  uint4 v;
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n mov.u32 %0, 0;\n mov.u32 %1, 0;\n mov.u32 %2, 0;\n mov.u32 %3, 0;\n"
+      " @q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w)
+      : "l"(p), "r"(unsigned(ok))
+      : "memory");
+  return v;
+}
+__device__ __forceinline__ void st16_if(bool ok, void* p, uint4 v) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %5, 0;\n @q st.global.v4.u32 [%4], {%0,%1,%2,%3};\n}" ::"r"(v.x), "r"(v.y),
+               "r"(v.z), "r"(v.w), "l"(p), "r"(unsigned(ok))
+               : "memory");
+}
 // streaming variants for data that is touched once
 __device__ __forceinline__ uint4 ld16_stream(const void* p) {
   uint4 v;
@@ -149,24 +169,72 @@ __device__ __forceinline__ uint4 ld16_stream(const void* p) {
   return v;
 }
 
-// dst[0,n) = src[0,n); any alignment. The fast path needs both 16-byte aligned.
+// Bytes s .. s+15 of the 32 bytes a, b (0 <= s < 16).
+__device__ __forceinline__ uint4 bytes_of_pair(uint4 a, uint4 b, unsigned s) {
+  unsigned w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int k = 0; k < 6; ++k) w[k] = (s & 8u) ? w[k + 2] : w[k];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) w[k] = (s & 4u) ? w[k + 1] : w[k];
+  const unsigned bits = (s & 3u) * 8u;
+  return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits),
+                    __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
+}
+
+// The thread's index, read anew: what is computed from it is not hoisted out of the loop over a
+// kernel's steps, where the address arithmetic of every phase together would not fit the registers.
+__device__ __forceinline__ unsigned fresh_tid() {
+  unsigned t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
+// dst[0,n) = src[0,n); any alignment. Whole 16-byte vectors of dst are stored; where src lies at
+// another offset within its vectors, each one is cut out of the two aligned vectors it spans (the
+// second is the neighbour lane's first, so it comes from L1). Byte by byte this was bound by the
+// number of loads: 8 ranks exchanging blocks of about 1 MiB at odd offsets, 1767 us against
+// 80 us a call on one B200.
+// A warp moves runs of eight (four) times 512 bytes, so that the loads of a run differ by a constant
+// and eight are in flight per thread. A share of 64 GiB or more does not occur.
 __device__ inline void cta_copy(char* dst, const char* src, size_t n) {
-  const int t = threadIdx.x, nt = blockDim.x;
-  if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0) {
-    const size_t nv = n >> 4;
-    size_t i = t;
-    for (; i + 7 * size_t(nt) < nv; i += 8 * size_t(nt)) {  // eight loads in flight per thread
-      uint4 r[8];
+  const unsigned t = fresh_tid(), lane = t & 31u, warp = t >> 5, warps = blockDim.x >> 5;
+  unsigned head = unsigned(-reinterpret_cast<intptr_t>(dst)) & 15u;
+  if (head > n) head = unsigned(n);
+  if (t < head) dst[t] = src[t];
+  dst += head;
+  src += head;
+  n -= head;
+  const unsigned nv = unsigned(n >> 4), tail = unsigned(n) & 15u;
+  const unsigned s = unsigned(reinterpret_cast<uintptr_t>(src) & 15u);
+  if (s == 0) {
+    constexpr int U = 8;
+    for (unsigned i = warp * (32 * U) + lane; i < nv; i += warps * (32 * U)) {
+      const char* from = src + (size_t(i) << 4);
+      char* to = dst + (size_t(i) << 4);
+      const unsigned left = nv - i;
+      uint4 r[U];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) r[u] = ld16(src + ((i + u * size_t(nt)) << 4));
+      for (int u = 0; u < U; ++u) r[u] = ld16_if(u * 32 < left, from + u * 512);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) st16(dst + ((i + u * size_t(nt)) << 4), r[u]);
+      for (int u = 0; u < U; ++u) st16_if(u * 32 < left, to + u * 512, r[u]);
     }
-    for (; i < nv; i += nt) st16(dst + (i << 4), ld16(src + (i << 4)));
-    for (size_t k = (nv << 4) + t; k < n; k += nt) dst[k] = src[k];
-    return;
+  } else {
+    constexpr int U = 4;
+    for (unsigned i = warp * (32 * U) + lane; i < nv; i += warps * (32 * U)) {
+      const char* from = src - s + (size_t(i) << 4);
+      char* to = dst + (size_t(i) << 4);
+      const unsigned left = nv - i;
+      uint4 r[U], q[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        r[u] = ld16_if(u * 32 < left, from + u * 512);
+        q[u] = ld16_if(u * 32 < left, from + u * 512 + 16);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) st16_if(u * 32 < left, to + u * 512, bytes_of_pair(r[u], q[u], s));
+    }
   }
-  for (size_t k = t; k < n; k += nt) dst[k] = src[k];
+  if (t < tail) dst[(size_t(nv) << 4) + t] = src[(size_t(nv) << 4) + t];
 }
 
 __device__ __forceinline__ void mc_st16(char* mc_addr, uint4 v) {
@@ -360,6 +428,155 @@ __device__ __forceinline__ Vec16<e4m3> apply_lanes<e4m3>(const Vec16<e4m3>& a, c
 template <>
 __device__ __forceinline__ Vec16<e5m2> apply_lanes<e5m2>(const Vec16<e5m2>& a, const Vec16<e5m2>& b, int op) {
   return apply_lanes_fp8<e5m2>(a, b, op);
+}
+
+// ---- Sum and Prod without the rare cases -----------------------------------------------------------
+// What the element rules add to a plain sum or product concerns NaN (whose payload survives, which
+// code it gets) and, for the 8-bit floats, overflow. Lanes<T> computes the plain form in the widest
+// instructions there are and sets `odd` when some lane may need more; the caller then takes the
+// whole vector through the rule (apply, apply_lanes). Acc holds the lanes as the chain of
+// combinations needs them: the vector itself, or, for the 8-bit floats, the f16 values of the codes,
+// so that a fold decodes every input once and its running value never.
+//
+// The packed 16-bit forms round once where the rule rounds to fp32 and then to the type. Both give
+// the same bits: an intermediate of q bits is innocuous for + and x from p-bit operands when
+// q >= 2p + 1 and q >= 2p (Figueroa, "When is double rounding innocuous?", 1995), here 24 against
+// p = 11 (fp16) and 8 (bf16), and the exact result of the operands' grids is representable in the
+// intermediate wherever the result is subnormal. The same holds for the 8-bit floats in f16:
+// 11 against p = 4 (e4m3) and 3 (e5m2); their products have at most 8 bits and are exact in f16
+// or lie below a quarter of the smallest code, and what overflows f16 overflows them.
+template <typename T>
+struct Lanes {
+  using Acc = Vec16<T>;
+  static __device__ __forceinline__ Acc open(const Vec16<T>& v) { return v; }
+  static __device__ __forceinline__ Vec16<T> close(const Acc& a) { return a; }
+  template <int kOp>
+  static __device__ __forceinline__ Acc combine(const Acc& a, const Acc& b, bool& odd) {
+    Acc r;
+#pragma unroll
+    for (int l = 0; l < int(16 / sizeof(T)); ++l) {
+      if constexpr (std::is_floating_point<T>::value) {
+        r.e[l] = kOp == kSum ? add_rn(a.e[l], b.e[l]) : mul_rn(a.e[l], b.e[l]);
+        odd |= r.e[l] != r.e[l];
+      } else {
+        r.e[l] = apply(a.e[l], b.e[l], kOp);
+      }
+    }
+    return r;
+  }
+};
+// f16 / bf16: two lanes per instruction; kInf is the type's infinity in both halves, so a magnitude
+// above it (NaN) carries into the sign bits of the sum below.
+template <typename T, unsigned kInf>
+struct PackedLanes {
+  using Acc = Vec16<T>;
+  static __device__ __forceinline__ Acc open(const Vec16<T>& v) { return v; }
+  static __device__ __forceinline__ Vec16<T> close(const Acc& a) { return a; }
+  template <int kOp>
+  static __device__ __forceinline__ Acc combine(const Acc& a, const Acc& b, bool& odd) {
+    const unsigned wa[4] = {a.raw.x, a.raw.y, a.raw.z, a.raw.w}, wb[4] = {b.raw.x, b.raw.y, b.raw.z, b.raw.w};
+    unsigned r[4], nan = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if constexpr (std::is_same<T, f16>::value) {
+        if constexpr (kOp == kSum) asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r[k]) : "r"(wa[k]), "r"(wb[k]));
+        else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r[k]) : "r"(wa[k]), "r"(wb[k]));
+      } else {
+        if constexpr (kOp == kSum) asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(r[k]) : "r"(wa[k]), "r"(wb[k]));
+        else asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r[k]) : "r"(wa[k]), "r"(wb[k]));
+      }
+      nan |= (r[k] & 0x7fff7fffu) + (0x7fff7fffu - kInf);
+    }
+    odd |= (nan & 0x80008000u) != 0;
+    Acc out;
+    out.raw = make_uint4(r[0], r[1], r[2], r[3]);
+    return out;
+  }
+};
+template <>
+struct Lanes<f16> : PackedLanes<f16, 0x7c007c00u> {};
+template <>
+struct Lanes<bf16> : PackedLanes<bf16, 0x7f807f80u> {};
+
+// e4m3 / e5m2: 16 lanes as eight f16 pairs plus the codes they stand for. The saturating encoder
+// gives the rule's code except above the largest finite value and for NaN; such lanes carry a code of
+// at least kTop (the largest finite code) or the hardware's NaN, and set `odd`.
+template <typename F8, unsigned kTop>
+struct Fp8Lanes {
+  struct Acc {
+    unsigned h[8];
+    uint4 codes;
+  };
+  static __device__ __forceinline__ unsigned decode(unsigned short two) {
+    unsigned pair;
+    if constexpr (std::is_same<F8, e4m3>::value) asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(pair) : "h"(two));
+    else asm("cvt.rn.f16x2.e5m2x2 %0, %1;" : "=r"(pair) : "h"(two));
+    return pair;
+  }
+  static __device__ __forceinline__ unsigned encode(unsigned pair) {
+    unsigned short two;
+    if constexpr (std::is_same<F8, e4m3>::value) asm("cvt.rn.satfinite.e4m3x2.f16x2 %0, %1;" : "=h"(two) : "r"(pair));
+    else asm("cvt.rn.satfinite.e5m2x2.f16x2 %0, %1;" : "=h"(two) : "r"(pair));
+    return two;
+  }
+  static __device__ __forceinline__ Acc open(const Vec16<F8>& v) {
+    Acc a;
+    a.codes = v.raw;
+    const unsigned w[4] = {v.raw.x, v.raw.y, v.raw.z, v.raw.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      a.h[2 * k] = decode(static_cast<unsigned short>(w[k] & 0xffffu));
+      a.h[2 * k + 1] = decode(static_cast<unsigned short>(w[k] >> 16));
+    }
+    return a;
+  }
+  static __device__ __forceinline__ Vec16<F8> close(const Acc& a) {
+    Vec16<F8> v;
+    v.raw = a.codes;
+    return v;
+  }
+  template <int kOp>
+  static __device__ __forceinline__ Acc combine(const Acc& a, const Acc& b, bool& odd) {
+    unsigned w[4], top = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      unsigned s[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if constexpr (kOp == kSum) asm("add.rn.f16x2 %0, %1, %2;" : "=r"(s[h]) : "r"(a.h[2 * k + h]), "r"(b.h[2 * k + h]));
+        else asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(s[h]) : "r"(a.h[2 * k + h]), "r"(b.h[2 * k + h]));
+      w[k] = encode(s[0]) | (encode(s[1]) << 16);
+      top |= (w[k] & 0x7f7f7f7fu) + (0x80u - kTop) * 0x01010101u;
+    }
+    odd |= (top & 0x80808080u) != 0;
+    Vec16<F8> v;
+    v.raw = make_uint4(w[0], w[1], w[2], w[3]);
+    return open(v);
+  }
+};
+template <>
+struct Lanes<e4m3> : Fp8Lanes<e4m3, 0x7eu> {};
+template <>
+struct Lanes<e5m2> : Fp8Lanes<e5m2, 0x7bu> {};
+
+// apply for every lane, any operator
+template <typename T>
+__device__ __forceinline__ Vec16<T> combine_lanes(const Vec16<T>& a, const Vec16<T>& b, int op) {
+  using L = Lanes<T>;
+  bool odd = false;
+  Vec16<T> out;
+  if (op == kSum)
+    out = L::close(L::template combine<kSum>(L::open(a), L::open(b), odd));
+  else if (op == kProd)
+    out = L::close(L::template combine<kProd>(L::open(a), L::open(b), odd));
+  else
+    return apply_lanes(a, b, op);
+  return odd ? apply_lanes(a, b, op) : out;
+}
+// value * scalar for every lane under the Prod rule
+template <typename T>
+__device__ __forceinline__ Vec16<T> scale_lanes(const Vec16<T>& v, T k) {
+  return combine_lanes(v, splat(k), kProd);
 }
 
 }  // namespace hx

@@ -73,8 +73,8 @@ __device__ inline void ring_pass(char* d0, char* d1, const char* own, const char
   auto lanes = [&](const Vec16<T>& x_own, const Vec16<T>& x_arr) -> Vec16<T> {  // `one` for 16 bytes
     Vec16<T> v;
     if (kOwn) {
-      v = r.premul ? apply_lanes(x_own, splat(r.scalar), kProd) : x_own;
-      if (kArr) v = apply_lanes(v, x_arr, r.op);
+      v = r.premul ? scale_lanes(x_own, r.scalar) : x_own;
+      if (kArr) v = combine_lanes(v, x_arr, r.op);
     } else {
       v = x_arr;
     }

@@ -85,7 +85,7 @@ struct RolesGeom {
   __device__ size_t buf(int step) const { return base0 + size_t(step % kRing) * buf_bytes; }
 };
 
-template <typename T>
+template <typename T, int kN>
 struct TwoShotRoleOps {
   const TwoShotArgs& a;
   FoldShared& sh;
@@ -98,17 +98,18 @@ struct TwoShotRoleOps {
   __device__ void stage_in(int k) {
     const WinView& w = a.w;
     const size_t step0 = size_t(k) * w.n * g.slice, buf = g.buf(k);
-    for (int jj = 1; jj < w.n; ++jj) {
-      const int j = (w.rank + jj) % w.n;
+    __syncthreads();  // the previous step is done with the table
+    if (threadIdx.x + 1 < unsigned(w.n)) {
+      const int j = (w.rank + 1 + int(threadIdx.x)) % w.n;
       const size_t lo = step0 + size_t(j) * g.slice + g.in_slice;
-      if (lo >= a.bytes) continue;
-      const size_t len = min_sz(a.sub_bytes, a.bytes - lo);
-      char* to = w.win[j] + buf + size_t(w.rank) * g.slice + g.in_slice;
-      if (a.fold.premul)
-        cta_scale_copy<T>(to, a.send + lo, len, scalar);
-      else
-        cta_copy(to, a.send + lo, len);
+      sh.piece_src[threadIdx.x] = a.send + lo;
+      sh.piece_dst[threadIdx.x] = w.win[j] + buf + size_t(w.rank) * g.slice + g.in_slice;
+      sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
+    if (a.fold.premul)
+      cta_pieces(sh, w.n - 1, a.sub_bytes, ScaleMover<T>{scalar});
+    else
+      cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover{});
   }
   __device__ void combine(int k) {
     const WinView& w = a.w;
@@ -126,27 +127,29 @@ struct TwoShotRoleOps {
       sh.mc_dst = a.use_mc ? w.mc + buf + g.second + size_t(me) * g.slice + g.in_slice : nullptr;
     __syncthreads();
     if (lo < a.bytes)
-      cta_fold<T>(a.recv + lo, sh, n - 1, min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold, me, n, scalar);
+      cta_fold<T, kN>(a.recv + lo, sh, n - 1, min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold, a.fold.premul != 0, me, n, scalar);
   }
   __device__ void stage_out(int k) {
     const WinView& w = a.w;
     const size_t step0 = size_t(k) * w.n * g.slice, buf = g.buf(k);
-    for (int ii = 1; ii < w.n; ++ii) {
-      const int i = (w.rank + ii) % w.n;
+    __syncthreads();  // the previous step is done with the table
+    if (threadIdx.x + 1 < unsigned(w.n)) {
+      const int i = (w.rank + 1 + int(threadIdx.x)) % w.n;
       const size_t lo = step0 + size_t(i) * g.slice + g.in_slice;
-      if (lo >= a.bytes) continue;
-      cta_copy(a.recv + lo, w.win[w.rank] + buf + g.second + size_t(i) * g.slice + g.in_slice,
-               min_sz(a.sub_bytes, a.bytes - lo));
+      sh.piece_src[threadIdx.x] = w.win[w.rank] + buf + g.second + size_t(i) * g.slice + g.in_slice;
+      sh.piece_dst[threadIdx.x] = a.recv + lo;
+      sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
+    cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover{});
   }
 };
 
-template <typename T>
+template <typename T, int kN>
 __device__ void twoshot_roles_body(const TwoShotArgs& a, int cta, int ncta, FoldShared& sh) {
   const int lanes = ncta / 3, lane = cta / 3, role = cta % 3;
   if (lane >= lanes) return;
   if (a.fold.kind == kFoldLinear && a.fold.ring) fill_ring_bounds(sh, a.fold.ring_count, a.w.n);
-  TwoShotRoleOps<T> ops(a, sh, lanes, lane);
+  TwoShotRoleOps<T, kN> ops(a, sh, lanes, lane);
   roles_pipeline(ops, a.w, a.epoch0, a.steps, lane, role, &sh.fail);
 }
 

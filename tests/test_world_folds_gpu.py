@@ -1,0 +1,129 @@
+"""The vector loops of the folds and copies where they can go wrong: every pair of 8-bit float
+codes and every 16-bit code against awkward partners, every rank count that has a loop of its own,
+blocks that end inside a vector, buffers at any element offset. Compared bit for bit with the host
+schedules (hxccl_b200.ops.oracle)."""
+import numpy as np
+import pytest
+
+from hxccl_b200 import _lib as L
+from hxccl_b200.ops import oracle
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def worlds():
+    from hxccl_b200.ops.world import World
+
+    made = {}
+
+    def get(n):
+        if n not in made:
+            made[n] = World(n, window_mb=8, wait_ms=20000)
+        return made[n]
+
+    yield get
+    for w in made.values():
+        w.close()
+
+
+def dev(a, shift=0):
+    """`a` on the GPU, `shift` bytes behind a 256-byte boundary"""
+    raw = torch.zeros(a.nbytes + 256, dtype=torch.uint8, device="cuda")
+    out = raw[shift:shift + a.nbytes]
+    out.copy_(torch.from_numpy(a.view(np.uint8).copy()))
+    return out
+
+
+def back(t, dt):
+    return t.cpu().numpy().view(oracle.raw_dtype(dt))
+
+
+def pairs(dt):
+    if L.DTYPE_SIZE[dt] == 1:
+        a, b = np.meshgrid(np.arange(256, dtype=np.uint8), np.arange(256, dtype=np.uint8))
+        return a.ravel().copy(), b.ravel().copy()
+    special = np.array([0, 1, 2, 0x3ff, 0x400, 0x7bff, 0x7c00, 0x7c01, 0x7e00, 0x7f7f, 0x7f80, 0x7f81, 0x7fff, 0x3c00, 0x3f80, 0x3555],
+                       dtype=np.uint16)
+    special = np.concatenate([special, special | 0x8000])
+    codes = np.arange(65536, dtype=np.uint16)
+    return np.tile(codes, len(special)), np.repeat(special, len(codes))
+
+
+@pytest.mark.parametrize("dt", [L.FLOAT8E4M3, L.FLOAT8E5M2, L.FLOAT16, L.BFLOAT16])
+def test_every_code_of_the_narrow_types(worlds, dt):
+    w = worlds(2)
+    a, b = pairs(dt)
+    for op in (L.SUM, L.PROD, L.MAX):
+        for variant, order in ((1, 0), (1, 1), (6, 0)):
+            w.tune(variant=variant, exact=True)
+            send = [dev(a), dev(b)]
+            recv = [torch.zeros_like(s) for s in send]
+            w.all_reduce(send, recv, len(a), dt, op=op, order=order)
+            torch.cuda.synchronize()
+            want = oracle.allreduce([a, b], dt, op, order=order)
+            for r in range(2):
+                assert np.array_equal(back(recv[r], dt), want[r]), (dt, op, variant, order, r)
+    w.tune(variant=0, exact=True)
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 6, 7, 8])
+def test_rank_counts_block_ends_and_offsets(worlds, n):
+    w = worlds(n)
+    rng = np.random.default_rng(n)
+    for dt in (L.FLOAT32, L.BFLOAT16, L.FLOAT8E4M3, L.INT32):
+        es = L.DTYPE_SIZE[dt]
+        for op in (L.SUM, L.AVG, L.MAX):
+            # blocks shorter than a vector, ends inside vectors, several runs per warp
+            for count in (n + 1, 16 * n + 3, 70001):
+                xs = [rng.integers(0, 256, count * es, dtype=np.uint8).view(oracle.raw_dtype(dt)) for _ in range(n)]
+                for shift in (0, es, 5 * es):
+                    for variant, order in ((1, 0), (1, 1), (2, 0)):
+                        w.tune(variant=variant, exact=True)
+                        buf = [dev(x, shift) for x in xs]
+                        w.all_reduce(buf, buf, count, dt, op=op, order=order)
+                        torch.cuda.synchronize()
+                        want = oracle.allreduce(xs, dt, op, order=order)
+                        for r in range(n):
+                            assert np.array_equal(back(buf[r], dt), want[r]), (n, dt, op, count, shift, variant, order, r)
+            # ReduceScatter of odd blocks: every rank's own input lies at another offset; in place as well
+            per = 4099
+            xs = [rng.integers(0, 256, per * n * es, dtype=np.uint8).view(oracle.raw_dtype(dt)) for _ in range(n)]
+            send = [dev(x) for x in xs]
+            recv = [torch.zeros(per * es, dtype=torch.uint8, device="cuda") for _ in range(n)]
+            w.reduce_scatter(send, recv, per, dt, op=op)
+            own = [send[r][r * per * es:(r + 1) * per * es] for r in range(n)]
+            w.reduce_scatter(send, own, per, dt, op=op)
+            torch.cuda.synchronize()
+            want = oracle.reducescatter(xs, dt, op)
+            for r in range(n):
+                assert np.array_equal(back(recv[r], dt), want[r]), ("rs", n, dt, op, r)
+                assert np.array_equal(back(own[r].contiguous(), dt), want[r]), ("rs in place", n, dt, op, r)
+    w.tune(variant=0, exact=True)
+    assert all(w.status(r) == (0, 0) for r in range(n))
+
+
+@pytest.mark.parametrize("dt", [L.FLOAT32, L.BFLOAT16, L.FLOAT8E5M2, L.INT64])
+def test_one_rank_scales(dt):
+    """Avg and PreMulSum over one rank: one scaling pass, any alignment, in place and out of place."""
+    import hxccl_b200 as hx
+
+    torch.zeros(1, device="cuda")
+    comm = hx.Communicator.init_rank(hx.get_unique_id(), 1, 0)
+    from hxccl_b200.ops.world import World
+
+    rng = np.random.default_rng(dt)
+    tdt = {L.FLOAT32: torch.float32, L.BFLOAT16: torch.bfloat16, L.FLOAT8E5M2: torch.float8_e5m2, L.INT64: torch.int64}[dt]
+    es = L.DTYPE_SIZE[dt]
+    with World(1, window_mb=4, wait_ms=20000) as w:  # the kernels' own one-rank form
+        for count in (1, 15, 128, 129, 300007):
+            x = rng.integers(0, 256, count * es, dtype=np.uint8).view(oracle.raw_dtype(dt))
+            for shift in (0, es):
+                a, out, ref = dev(x, shift), dev(np.zeros_like(x), shift), dev(np.zeros_like(x))
+                comm.all_reduce(a.view(tdt), out.view(tdt), op=hx.AVG)
+                w.all_reduce([a], [ref], count, dt, op=L.AVG)
+                comm.all_reduce(a.view(tdt), a.view(tdt), op=hx.AVG)
+                torch.cuda.synchronize()
+                assert torch.equal(out, ref) and torch.equal(a, ref), (dt, count, shift)
+    comm.destroy()
