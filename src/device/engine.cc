@@ -22,6 +22,12 @@ LaunchShape Engine::shape(const Geometry& g) const {
   return LaunchShape{g.ctas, g.threads, world() ? int(views.size()) : 0};
 }
 
+Tuning Engine::lean(const Tuning& t) const {
+  Tuning out = t;
+  if (world_lean) out.max_ctas = std::min(2 * t.max_ctas, kMaxCtas);
+  return out;
+}
+
 cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpPlan& plan,
                               int order, cudaStream_t st) {
   const size_t bytes = count * dtype_size(dt);
@@ -87,7 +93,7 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
   }
   if (var == kVarRing) {
     const size_t es = dtype_size(dt);
-    const Geometry g = plan_ring((count + n() - 1) / n() * es, n(), views[0].half_bytes, tune);
+    const Geometry g = plan_ring((count + n() - 1) / n() * es, n(), views[0].half_bytes, lean(tune));
     HX_CHECK_PLAN(kPlanRing, g, (count + n() - 1) / n() * es);
     std::vector<TwoShotArgs> args(views.size());
     for (size_t r = 0; r < views.size(); ++r)
@@ -146,7 +152,7 @@ cudaError_t Engine::reducescatter(const RankBufs* b, size_t per, int dt, const O
                         : ((this->tune.rs_ring_min && block * n() >= this->tune.rs_ring_min) || forced_variant == kVarRing);
   const Tuning tune = with_row(this->tune, row, ring ? kVarRing : kVarOneShot);
   if (n() >= 2 && block > 0 && ring) {
-    const Geometry g = plan_ring(block, n(), views[0].half_bytes, tune, true);
+    const Geometry g = plan_ring(block, n(), views[0].half_bytes, lean(tune), true);
     HX_CHECK_PLAN(kPlanRingRs, g, block);
     std::vector<TwoShotArgs> args(views.size());
     for (size_t r = 0; r < views.size(); ++r)
@@ -178,7 +184,7 @@ cudaError_t Engine::reduce(const RankBufs* b, size_t count, int dt, const OpPlan
 }
 
 #define HX_COPY_COLLECTIVE(MAXPAIR, BUILD)                                  \
-  const Geometry g = plan_xchg(MAXPAIR, n(), views[0].half_bytes, tune);    \
+  const Geometry g = plan_xchg(MAXPAIR, n(), views[0].half_bytes, lean(tune)); \
   HX_CHECK_PLAN(kPlanXchg, g, MAXPAIR);                                     \
   std::vector<XchgArgs> args(views.size());                                 \
   for (size_t r = 0; r < views.size(); ++r) { BUILD; }                      \
@@ -251,16 +257,30 @@ cudaError_t Engine::p2p(const RankP2p* ops, cudaStream_t st) {
   // when lanes x kP2pWorkers CTAs do not fit, one CTA serves several workers of its lane one
   // after the other (both ends of a lane walk them in the same order, so the pairing holds).
   const int sharing = world() ? int(nr) : 1;
-  const int most_lanes = std::max(1, std::min(kMaxLanes, 2 * (n() - 1)));
+  int most_lanes = std::max(1, std::min(kMaxLanes, 2 * (n() - 1)));
+  if (world()) {  // this process sees the lanes of every rank: count them
+    most_lanes = 1;
+    for (size_t r = 0; r < nr; ++r) {
+      bool seen[2][kMaxRanks] = {};
+      int lanes = 0;
+      for (const P2pOp& o : left[r]) {
+        bool& s = seen[o.is_send ? 1 : 0][o.peer];
+        lanes += s ? 0 : 1;
+        s = true;
+      }
+      most_lanes = std::max(most_lanes, std::min(lanes, kMaxLanes));
+    }
+  }
   auto workers_per_cta = [&](int width) {
-    const int resident = max_resident_ctas(width) / sharing;
+    // k_p2p_world keeps two 512-thread CTAs on an SM (its launch bounds)
+    const int resident = max_resident_ctas(world() ? 256 : width) / sharing;
     int wpc = 1;
     while (wpc < kP2pWorkers && most_lanes * (kP2pWorkers / wpc) > resident) wpc *= 2;
     return most_lanes * (kP2pWorkers / wpc) <= resident ? wpc : 0;
   };
-  int threads = world() ? 256 : tune.p2p_threads;
+  int threads = world() ? 512 : tune.p2p_threads;
   int wpc = workers_per_cta(threads);
-  if (threads == 512 && wpc != 1) {  // narrower CTAs: twice as many are resident
+  if (threads == 512 && wpc != 1 && !world()) {  // narrower CTAs: twice as many are resident
     const int narrow = workers_per_cta(256);
     if (narrow && (!wpc || narrow < wpc)) threads = 256, wpc = narrow;
   }

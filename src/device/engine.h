@@ -34,6 +34,10 @@ class Engine {
   std::vector<WinView> views;
   Tuning tune;
   uint64_t epoch = 2;  // flags start at zero; the first step must be able to tell
+  // World: kernels compiled for two 512-thread CTAs per SM (copies, ring, lanes) may launch twice the
+  // grid of the others; off once the caller has set a grid limit.
+  bool world_lean = false;
+  Tuning lean(const Tuning& t) const;
   int forced_variant = kVarAuto;
   int last_variant = kVarAuto;  // what the latest AllReduce used
   unsigned long long launches = 0;  // kernels launched so far

@@ -50,10 +50,11 @@ bool make_plan(int n, int dt, int op, const void* scalar, OpPlan* p) {
   return true;
 }
 
-// CTAs the whole world may use together. Kept well below the co-residency bound of the
-// heaviest kernel: a cooperative launch is refused outright when it does not fit, and other
-// work on the device can take SMs away.
-int world_cta_budget() { return std::max(1, max_resident_ctas(512) * 3 / 4); }
+// CTAs the whole world may use together: one 512-thread CTA per SM, which every kernel fits
+// (max_resident_ctas). A cooperative launch waits until they all fit; it is refused only when the
+// device could never hold them. Leaving a quarter of the SMs free, 8 ranks, 16 MiB e4m3: 155 us
+// against 135 us; 7 ranks, 28 MB fp32 average: 261 us against 197 us.
+int world_cta_budget() { return std::max(1, max_resident_ctas(512)); }
 
 std::vector<RankBufs> bufs(hxcclWorld* w, const void* const* send, void* const* recv) {
   std::vector<RankBufs> b(w->n);
@@ -97,16 +98,29 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
     v.half_off[0] = kHeaderBytes + p2p;
     v.half_off[1] = v.half_off[0] + half;
     v.half_bytes = half;
-    v.p2p_slot = kP2pSlotBytes;
+    v.p2p_slot = kP2pSlotBytes / 2;  // 4 ranks, ring shift of 32 MiB: 100 us with 512 KiB slots, 95 with 256, 114 with 128
     v.wait_ns = uint64_t(wait_ms) * 1000000ull;
     v.rank = r;
     v.n = n;
     w->eng.views.push_back(v);
   }
   // the whole world must be co-resident: a cooperative launch refuses anything larger
-  w->eng.tune.max_ctas = std::max(1, std::min(64, world_cta_budget() / n));
+  w->eng.tune.max_ctas = std::max(1, std::min(kMaxCtas, world_cta_budget() / n));
+  w->eng.world_lean = true;
   w->eng.tune.threads = 512;  // one CTA per SM: the budget above counts on it
   w->eng.tune.roles_min_ranks = 2;
+  // Where the lines lie when all ranks share one GPU (one B200, us a call, fp32 sum):
+  //   lines up to 64 KiB      8 ranks, 40 KiB bf16: lines 16.3, one-shot 17.1; 8 ranks, 256 KiB: 28.1 and 16.9
+  //   4 KiB grain             8 ranks, 512 KiB two-shot: 17.2, with 16 KiB 22.4; 1 MiB 19.3 and 23.1
+  //   ring from 48 MiB        2 ranks, 64 MiB: ring 93, two-shot 119; 16 MiB: 40 and 32; 8 ranks, 64 MiB: 425 and
+  //                           511, 16 MiB: 144 and 133. Never the role pipeline: 16 MiB on 4 ranks 152, two-shot 86
+  //   hops of 64 KiB on two ranks (256 MiB: 289; 128 KiB: 311; 512 KiB: 366), 128 KiB on more (4 ranks,
+  //                           64 MiB: 206; 64 KiB: 220): the slots of all CTAs then stay in L2
+  w->eng.tune.ll_max = 64 * 1024;
+  w->eng.tune.grain = 4 * 1024;
+  w->eng.tune.ring_min = 48u << 20;
+  w->eng.tune.roles_min = ~size_t(0);
+  w->eng.tune.ring_sub = (n == 2 ? 64 : 128) * 1024;
   *out = w;
   return cudaDeviceSynchronize() == cudaSuccess ? hxcclSuccess : hxcclUnhandledCudaError;
 }
@@ -126,13 +140,17 @@ hxcclResult_t hxcclWorldTune(hxcclWorld_t w, int variant, int exact, int max_cta
   if (!w) return hxcclInvalidArgument;
   w->eng.forced_variant = variant;
   w->eng.tune.exact = exact != 0;
-  if (max_ctas > 0) w->eng.tune.max_ctas = std::min(max_ctas, std::max(1, world_cta_budget() / w->n));
+  if (max_ctas > 0) {
+    w->eng.tune.max_ctas = std::min(max_ctas, std::max(1, world_cta_budget() / w->n));
+    w->eng.world_lean = false;
+  }
   return hxcclSuccess;
 }
 
 hxcclResult_t hxcclWorldTuneKnob(hxcclWorld_t w, const char* name, long value) {
   if (!w) return hxcclInvalidArgument;
   if (!set_knob(&w->eng.tune, name, value)) return hxcclInvalidArgument;
+  if (std::strcmp(name, "max_ctas") == 0) w->eng.world_lean = false;
   w->eng.tune.max_ctas = std::min(w->eng.tune.max_ctas, std::max(1, world_cta_budget() / w->n));
   return hxcclSuccess;
 }

@@ -31,7 +31,7 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
   T scalar{};
   if (kFold) {
     if (a.fold.premul) scalar = load_scalar<T>(a.fold);
-    if (a.fold.kind == kFoldLinear && a.fold.ring) fill_ring_bounds(sh, a.fold.ring_count, n);
+    open_fold(sh, a.fold, me, n);
   }
   if (threadIdx.x == 0) sh.fail = 0;
   __syncthreads();
@@ -86,7 +86,7 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
       }
       if (threadIdx.x == 0) sh.mc_dst = nullptr;
       __syncthreads();
-      cta_fold<T, kN>(a.fold_dst + lo, sh, 0, len, a.fold_elem0 + lo / sizeof(T), a.fold, a.fold.premul != 0, me, n, scalar);
+      cta_fold<T, kN>(a.fold_dst + lo, sh, 0, len, a.fold_elem0 + lo / sizeof(T), a.fold.premul != 0, scalar);
     }
   };
 
@@ -134,8 +134,7 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
   const int me = w.rank, n = w.n;
   T scalar{};
   if (a.fold.premul) scalar = load_scalar<T>(a.fold);
-  if (a.fold.kind == kFoldLinear && a.fold.ring) fill_ring_bounds(sh, a.fold.ring_count, n);
-  if (threadIdx.x == 0) sh.fail = 0;
+  open_fold(sh, a.fold, me, n);
   __syncthreads();
   char* mine = w.win[me];
   const Staging stg(w, a.epoch0, a.steps);
@@ -189,7 +188,7 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
     __syncthreads();
     if (lo < a.bytes)  // kCast: every source is staged and already scaled; the result stays in the window
       cta_fold<T, kN>(kCast ? mine + buf + ag_base + size_t(me) * slice + in_slice : a.recv + lo, sh, n - 1,
-                  min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold, !kCast && a.fold.premul != 0, me, n, scalar);
+                  min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), !kCast && a.fold.premul != 0, scalar);
     __syncthreads();
     tm.lap(kTrMid);
     signal_all(w, kOffFlagsB, cta, e_step0 + step);

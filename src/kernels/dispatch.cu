@@ -13,7 +13,9 @@ __global__ void __launch_bounds__(512) k_xchg_copy(const __grid_constant__ XchgA
   __shared__ FoldShared sh;
   xchg_body<uint8_t, false>(a, blockIdx.x, gridDim.x, sh);
 }
-__global__ void __launch_bounds__(512) k_xchg_copy_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
+// Worlds run the copies, the lanes and the ring with two CTAs per SM (64 registers a thread suffice
+// there): 8 ranks, blocks of about 1 MiB at odd offsets: one CTA per SM 74 us, two 61 us.
+__global__ void __launch_bounds__(512, 2) k_xchg_copy_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
   __shared__ FoldShared sh;
   xchg_body<uint8_t, false>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
@@ -48,7 +50,7 @@ __global__ void __launch_bounds__(512) k_p2p_bulk(const __grid_constant__ P2pArg
   p2p_cta(a, &fail, &word, &pipe);
 }
 template <int kLanes, int kOps>
-__global__ void __launch_bounds__(512) k_p2p_world(const __grid_constant__ P2pWorldArgs<kLanes, kOps> a) {
+__global__ void __launch_bounds__(512, 2) k_p2p_world(const __grid_constant__ P2pWorldArgs<kLanes, kOps> a) {
   __shared__ int fail;
   __shared__ unsigned long long word;
   const int groups = kP2pWorkers / a.workers_per_cta, r = blockIdx.y;
@@ -132,6 +134,7 @@ static cudaError_t launch_p2p_world(const P2pArgs* args, LaunchShape s, cudaStre
   P2pWorldArgs<kLanes, kOps> a;
   static_assert(sizeof a <= 32764, "kernel parameters");
   if (s.world > kMaxRanks) return cudaErrorInvalidValue;
+  if (cudaError_t e = refuse_capture(st)) return e;
   int lane = 0, op = 0;
   a.workers_per_cta = args[0].workers_per_cta;
   for (int r = 0; r < s.world; ++r) {

@@ -27,8 +27,24 @@ struct FoldShared {
   const char* piece_src[kMaxRanks];  // pieces of the copy at hand (cta_pieces)
   char* piece_dst[kMaxRanks];
   size_t piece_len[kMaxRanks];
+  FoldSpec spec;  // of the launch (open_fold)
+  int rank, n;
   int fail;
 };
+
+// Once per kernel, by all threads; the caller's next barrier makes it visible. The phases below are
+// functions of their own (not inlined), so that each has the whole register budget to itself, and take
+// what the launch fixes from here rather than from the kernel's parameters.
+__device__ inline void fill_ring_bounds(FoldShared& sh, size_t count, int n);
+__device__ inline void open_fold(FoldShared& sh, const FoldSpec& f, int rank, int n) {
+  if (threadIdx.x == 0) {
+    sh.spec = f;
+    sh.rank = rank;
+    sh.n = n;
+    sh.fail = 0;
+  }
+  if (f.kind == kFoldLinear && f.ring) fill_ring_bounds(sh, f.ring_count, n);
+}
 
 // ring-block boundaries of `count` elements over n ranks, once per kernel
 __device__ inline void fill_ring_bounds(FoldShared& sh, size_t count, int n) {
@@ -99,8 +115,9 @@ __device__ __forceinline__ T fold_doubling_pow2(T (&x)[N], int op) {
 
 // One element through the general path: any fold kind, any rank count, any alignment.
 template <typename T>
-__device__ inline T fold_element(const FoldShared& sh, size_t e, size_t elem0, const FoldSpec& f, bool premul, int rank,
-                                 int n, T scalar) {
+__device__ inline T fold_element(const FoldShared& sh, size_t e, size_t elem0, bool premul, T scalar) {
+  const FoldSpec& f = sh.spec;
+  const int rank = sh.rank, n = sh.n;
   T x[kMaxRanks];
   for (int i = 0; i < n; ++i) x[i] = reinterpret_cast<const T*>(sh.src[i])[e];
   if (premul) x[rank] = scale(x[rank], scalar);
@@ -138,24 +155,19 @@ __device__ __forceinline__ void fold_store(char* dst, bool dst_aligned, const Fo
 // result, and with the sources in the order r ^ q they are a plain binary tree.
 template <typename T, int N, int U, int kOp, bool kTree>
 __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const FoldShared& sh, int nremote, unsigned v_lo,
-                                             unsigned v_hi, int first, const FoldSpec& f, bool premul, int rank, int n, T scalar) {
+                                             unsigned v_hi, int first, bool premul, T scalar) {
   using L = Lanes<T>;
+  const FoldSpec& f = sh.spec;
+  const int rank = sh.rank, n = kTree ? N : sh.n;
   constexpr int V = 16 / sizeof(T);
   const unsigned t = fresh_tid(), lane = t & 31u, warp = t >> 5, warps = blockDim.x >> 5;
-  const char* src[N];
-  int own = 0;
-#pragma unroll
-  for (int k = 0; k < N; ++k) {
-    int idx;
-    if constexpr (kTree) {
-      idx = rank ^ k;
-    } else {
-      idx = first + (f.dir < 0 ? n - k : k);
-      idx = idx >= n ? idx - n : idx;
-    }
-    src[k] = k < n ? sh.src[idx] : nullptr;
-    if (k < n && idx == rank) own = k;
-  }
+  // the rank whose value comes k-th; its address is read from shared memory where it is needed (eight
+  // pointers held over the loop cost sixteen registers)
+  auto rank_at = [&](int k) {
+    if constexpr (kTree) return rank ^ k;
+    const int idx = first + (f.dir < 0 ? n - k : k);
+    return idx >= n ? idx - n : idx;
+  };
   // window slots are aligned; this rank's own input need not be
   const unsigned shift = unsigned(reinterpret_cast<uintptr_t>(sh.src[rank]) & 15u);
   for (unsigned v0 = v_lo + warp * (32 * U) + lane; v0 < v_hi; v0 += warps * (32 * U)) {  // a warp takes runs of U x 512 bytes
@@ -163,7 +175,8 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
     Vec16<T> in[U][N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-      const char* p = src[k] + (size_t(v0) << 4) - (k == own ? shift : 0u);
+      const int idx = k < n ? rank_at(k) : rank;
+      const char* p = sh.src[idx] + (size_t(v0) << 4) - (idx == rank ? shift : 0u);
 #pragma unroll
       for (int u = 0; u < U; ++u) in[u][k].raw = ld16_if(u * 32 < left && k < n, p + u * 512);
     }
@@ -173,7 +186,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
         const uint4 next = ld16_if(u * 32 < left, sh.src[rank] + (size_t(v0) << 4) - shift + u * 512 + 16);
 #pragma unroll
         for (int k = 0; k < N; ++k)
-          if (k == own) in[u][k].raw = bytes_of_pair(in[u][k].raw, next, shift);
+          if (k < n && rank_at(k) == rank) in[u][k].raw = bytes_of_pair(in[u][k].raw, next, shift);
       }
     }
 #pragma unroll
@@ -198,14 +211,14 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
         for (int k = 0; k < N; ++k) {
           if (k >= n) continue;
           typename L::Acc x = L::open(in[u][k]);
-          if (premul && k == own) x = L::template combine<kProd>(x, L::open(splat(scalar)), odd);
+          if (premul && rank_at(k) == rank) x = L::template combine<kProd>(x, L::open(splat(scalar)), odd);
           acc = k == 0 ? x : L::template combine<kOp>(x, acc, odd);
         }
         out = L::close(acc);
       } else {
 #pragma unroll
         for (int k = 0; k < N; ++k)
-          if (premul && k == own) in[u][k] = apply_lanes(in[u][k], splat(scalar), kProd);
+          if (premul && k < n && rank_at(k) == rank) in[u][k] = apply_lanes(in[u][k], splat(scalar), kProd);
         if constexpr (kTree) {
 #pragma unroll
           for (int bit = 1; bit < N; bit <<= 1)
@@ -227,8 +240,8 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 #pragma unroll
           for (int k = 0; k < N; ++k) {
             if (k >= n) continue;
-            y[k] = reinterpret_cast<const T*>(src[k])[e];
-            if (premul && k == own) y[k] = scale(y[k], scalar);
+            y[k] = reinterpret_cast<const T*>(sh.src[rank_at(k)])[e];
+            if (premul && rank_at(k) == rank) y[k] = scale(y[k], scalar);
           }
           T r = y[0];
           if constexpr (kTree) {
@@ -267,13 +280,15 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 // kN = 0 (one rank, nine to sixteen ranks). Seven ranks, 28 MB fp32 average, on one B200: 677 us a call
 // when seven ranks took that general path, 243 us with the vector loop.
 template <typename T, int kN>
-__device__ __forceinline__ void cta_fold(char* dst, const FoldShared& sh, int nremote, size_t nbytes, size_t elem0,
-                                         const FoldSpec& f, bool premul, int rank, int n, T scalar) {
+static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, int nremote, size_t nbytes, size_t elem0,
+                                             bool premul, T scalar) {
+  const FoldSpec& f = sh.spec;
+  const int n = sh.n;
   constexpr int V = 16 / sizeof(T);
   const unsigned t = threadIdx.x, nt = blockDim.x;
   const unsigned total = unsigned(nbytes / sizeof(T));
   auto element = [&](unsigned e) {
-    const T r = fold_element<T>(sh, e, elem0, f, premul, rank, n, scalar);
+    const T r = fold_element<T>(sh, e, elem0, premul, scalar);
     reinterpret_cast<T*>(dst)[e] = r;
     for (int q = 0; q < nremote; ++q) reinterpret_cast<T*>(sh.remote[q])[e] = r;
   };
@@ -299,13 +314,13 @@ __device__ __forceinline__ void cta_fold(char* dst, const FoldShared& sh, int nr
       }
       if (tree) {
         if (f.op == kSum)
-          fold_vectors<T, kN, 1, kSum, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, f, premul, rank, n, scalar);
+          fold_vectors<T, kN, 1, kSum, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
         else
-          fold_vectors<T, kN, 1, -1, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, f, premul, rank, n, scalar);
+          fold_vectors<T, kN, 1, -1, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
       } else if (f.op == kSum) {
-        fold_vectors<T, kN, U, kSum, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, f, premul, rank, n, scalar);
+        fold_vectors<T, kN, U, kSum, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
       } else {
-        fold_vectors<T, kN, 1, -1, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, f, premul, rank, n, scalar);
+        fold_vectors<T, kN, 1, -1, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
       }
       v = v_hi;
     }
@@ -333,7 +348,7 @@ __device__ __forceinline__ void cta_pieces_one_by_one(const FoldShared& sh, int 
 // The caller has filled sh.piece_*[0..np) (threads below np, one each); no piece is longer than
 // `longest`. Called by all threads; begins with the barrier that makes the table visible.
 template <typename M>
-__device__ __forceinline__ void cta_pieces(const FoldShared& sh, int np, size_t longest, const M& m) {
+__device__ __forceinline__ void cta_pieces(const FoldShared& sh, int np, size_t longest, M m) {
   constexpr int U = M::kUnroll, V = 16 / sizeof(typename M::Elem);
   const unsigned t = fresh_tid(), lane = t & 31u, nt = blockDim.x;
   __syncthreads();

@@ -13,9 +13,10 @@ namespace hx {
 // of the 32 KB a launch may carry). Staged through device memory they cost a stream
 // synchronisation (an earlier launch might still read the buffer) and a pageable copy per call:
 // 8 ranks, 41 KB bf16: 34.3 us a call staged, 22.6 us as parameters; 8 ranks, 8 B: 19.0 and 15.2 us.
-template <typename Args>
+// Kernels made for up to kN ranks carry kN blocks only.
+template <typename Args, int kN = 0>
 struct WorldArgs {
-  Args rank[kMaxRanks];
+  Args rank[kN ? kN : kMaxRanks];
 };
 
 // kN: the rank count the fold is unrolled for (see cta_fold, fold.cuh); HX_BY_RANKS picks it.
@@ -25,7 +26,7 @@ __global__ void __launch_bounds__(512) k_xchg_fold(const __grid_constant__ XchgA
   xchg_body<T, true, kN>(a, blockIdx.x, gridDim.x, sh);
 }
 template <typename T, int kN>
-__global__ void __launch_bounds__(512) k_xchg_fold_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
+__global__ void __launch_bounds__(512) k_xchg_fold_world(const __grid_constant__ WorldArgs<XchgArgs, kN> a) {
   __shared__ FoldShared sh;
   xchg_body<T, true, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
@@ -35,7 +36,7 @@ __global__ void __launch_bounds__(512) k_twoshot(const __grid_constant__ TwoShot
   twoshot_body<T, kN>(a, blockIdx.x, gridDim.x, sh);
 }
 template <typename T, int kN>
-__global__ void __launch_bounds__(512) k_twoshot_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
+__global__ void __launch_bounds__(512) k_twoshot_world(const __grid_constant__ WorldArgs<TwoShotArgs, kN> a) {
   __shared__ FoldShared sh;
   twoshot_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(512) k_twoshot_cast(const __grid_constant__ Tw
   twoshot_body<T, kN, true>(a, blockIdx.x, gridDim.x, sh);
 }
 template <typename T, int kN>
-__global__ void __launch_bounds__(512) k_twoshot_cast_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
+__global__ void __launch_bounds__(512) k_twoshot_cast_world(const __grid_constant__ WorldArgs<TwoShotArgs, kN> a) {
   __shared__ FoldShared sh;
   twoshot_body<T, kN, true>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
@@ -58,7 +59,7 @@ __global__ void __launch_bounds__(512) k_twoshot_roles(const __grid_constant__ T
   twoshot_roles_body<T, kN>(a, blockIdx.x, gridDim.x, sh);
 }
 template <typename T, int kN>
-__global__ void __launch_bounds__(512) k_twoshot_roles_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
+__global__ void __launch_bounds__(512) k_twoshot_roles_world(const __grid_constant__ WorldArgs<TwoShotArgs, kN> a) {
   __shared__ FoldShared sh;
   twoshot_roles_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
@@ -69,27 +70,36 @@ __global__ void __launch_bounds__(512) k_ring(const __grid_constant__ TwoShotArg
   ring_body<T>(a, blockIdx.x, gridDim.x, sh);
 }
 template <typename T>
-__global__ void __launch_bounds__(512) k_ring_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
+__global__ void __launch_bounds__(512, 2) k_ring_world(const __grid_constant__ WorldArgs<TwoShotArgs> a) {
   __shared__ FoldShared sh;
   ring_body<T>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
-template <typename T>
+template <typename T, int kN>
 __global__ void __launch_bounds__(256, 1) k_ll(const __grid_constant__ LLArgs a) {
   __shared__ FoldShared sh;
-  ll_body<T>(a, blockIdx.x, gridDim.x, sh);
+  ll_body<T, kN>(a, blockIdx.x, gridDim.x, sh);
 }
-template <typename T>
-__global__ void __launch_bounds__(256, 1) k_ll_world(const __grid_constant__ WorldArgs<LLArgs> a) {
+template <typename T, int kN>
+__global__ void __launch_bounds__(256, 1) k_ll_world(const __grid_constant__ WorldArgs<LLArgs, kN> a) {
   __shared__ FoldShared sh;
-  ll_body<T>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
+  ll_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
-template <typename Args>
+// A world's call is refused on a stream that is being captured: its epochs are part of the launch,
+// and a replay would meet flags that are already up.
+inline cudaError_t refuse_capture(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &status);
+  return e == cudaSuccess && status != cudaStreamCaptureStatusNone ? cudaErrorStreamCaptureUnsupported : e;
+}
+
+template <int kN = 0, typename Args>
 cudaError_t launch_world(const void* kernel, const Args* args, LaunchShape s, cudaStream_t st) {
-  static_assert(sizeof(WorldArgs<Args>) <= 32764, "kernel parameters");
-  if (s.world > kMaxRanks) return cudaErrorInvalidValue;
-  WorldArgs<Args> all;  // blocks of ranks that do not exist stay unset: no CTA reads them
+  static_assert(sizeof(WorldArgs<Args, kN>) <= 32764, "kernel parameters");
+  if (s.world > (kN ? kN : kMaxRanks)) return cudaErrorInvalidValue;
+  if (cudaError_t e = refuse_capture(st)) return e;
+  WorldArgs<Args, kN> all;  // blocks of ranks that do not exist stay unset: no CTA reads them
   memcpy(all.rank, args, sizeof(Args) * size_t(s.world));
   void* params[] = {&all};
   return cudaLaunchCooperativeKernel(kernel, dim3(s.ctas, s.world), dim3(s.threads), params, 0, st);
@@ -97,7 +107,7 @@ cudaError_t launch_world(const void* kernel, const Args* args, LaunchShape s, cu
 
 // Launches KERNEL<T, kN>, or KERNEL_world<T, kN> for a world, for the rank count of args[0].
 #define HX_LAUNCH_RANKS(KERNEL, KN)                                                                       \
-  if (s.world) return launch_world(reinterpret_cast<const void*>(&KERNEL##_world<T, KN>), args, s, st);   \
+  if (s.world) return launch_world<KN>(reinterpret_cast<const void*>(&KERNEL##_world<T, KN>), args, s, st); \
   KERNEL<T, KN><<<s.ctas, s.threads, 0, st>>>(*args);                                                     \
   return cudaGetLastError()
 #define HX_BY_RANKS(KERNEL)                                                          \
@@ -133,9 +143,11 @@ cudaError_t launch_ring_t(const TwoShotArgs* args, LaunchShape s, cudaStream_t s
 
 template <typename T>
 cudaError_t launch_ll_t(const LLArgs* args, LaunchShape s, cudaStream_t st) {
-  if (s.world) return launch_world(reinterpret_cast<const void*>(&k_ll_world<T>), args, s, st);
-  k_ll<T><<<s.ctas, s.threads, 0, st>>>(*args);
-  return cudaGetLastError();
+  const int n = args[0].w.n;  // loops of a fixed length for 2, 4 and 8 ranks only
+  if (n == 2) { HX_LAUNCH_RANKS(k_ll, 2); }
+  if (n == 4) { HX_LAUNCH_RANKS(k_ll, 4); }
+  if (n == 8) { HX_LAUNCH_RANKS(k_ll, 8); }
+  HX_LAUNCH_RANKS(k_ll, 0);
 }
 
 // ---- standalone elementwise kernels --------------------------------------------------------

@@ -172,14 +172,9 @@ __device__ void ll_ranks(const LLArgs& a, int cta, int ncta, FoldShared& sh) {
   }
 }
 
-template <typename T>
-__device__ void ll_body(const LLArgs& a, int cta, int ncta, FoldShared& sh) {
-  switch (a.w.n) {
-    case 2: ll_ranks<T, 2>(a, cta, ncta, sh); break;
-    case 4: ll_ranks<T, 4>(a, cta, ncta, sh); break;
-    case 8: ll_ranks<T, 8>(a, cta, ncta, sh); break;
-    default: ll_ranks<T, kMaxRanks>(a, cta, ncta, sh); break;
-  }
+template <typename T, int kN>
+__device__ __forceinline__ void ll_body(const LLArgs& a, int cta, int ncta, FoldShared& sh) {
+  ll_ranks<T, kN ? kN : kMaxRanks>(a, cta, ncta, sh);
 }
 
 }  // namespace hx

@@ -127,7 +127,7 @@ struct TwoShotRoleOps {
       sh.mc_dst = a.use_mc ? w.mc + buf + g.second + size_t(me) * g.slice + g.in_slice : nullptr;
     __syncthreads();
     if (lo < a.bytes)
-      cta_fold<T, kN>(a.recv + lo, sh, n - 1, min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold, a.fold.premul != 0, me, n, scalar);
+      cta_fold<T, kN>(a.recv + lo, sh, n - 1, min_sz(a.sub_bytes, a.bytes - lo), lo / sizeof(T), a.fold.premul != 0, scalar);
   }
   __device__ void stage_out(int k) {
     const WinView& w = a.w;
@@ -148,7 +148,7 @@ template <typename T, int kN>
 __device__ void twoshot_roles_body(const TwoShotArgs& a, int cta, int ncta, FoldShared& sh) {
   const int lanes = ncta / 3, lane = cta / 3, role = cta % 3;
   if (lane >= lanes) return;
-  if (a.fold.kind == kFoldLinear && a.fold.ring) fill_ring_bounds(sh, a.fold.ring_count, a.w.n);
+  open_fold(sh, a.fold, a.w.rank, a.w.n);
   TwoShotRoleOps<T, kN> ops(a, sh, lanes, lane);
   roles_pipeline(ops, a.w, a.epoch0, a.steps, lane, role, &sh.fail);
 }

@@ -127,3 +127,31 @@ def test_one_rank_scales(dt):
                 torch.cuda.synchronize()
                 assert torch.equal(out, ref) and torch.equal(a, ref), (dt, count, shift)
     comm.destroy()
+
+
+def test_a_world_refuses_a_capturing_stream(worlds):
+    """The epochs of a world's launch are baked into its parameters, so a replay would be wrong: calls on
+    a capturing stream fail, and the world works on afterwards."""
+    from hxccl_b200.comm import HxcclError
+
+    w = worlds(2)
+    w.tune(variant=0, exact=True)
+    x = [torch.full((50000,), float(r + 1), device="cuda") for r in range(2)]
+    y = [torch.zeros_like(t) for t in x]
+    torch.cuda.synchronize()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin()
+        for call in (lambda: w.all_reduce(x, y, 50000, L.FLOAT32), lambda: w.all_reduce(x, y, 64, L.FLOAT32),
+                     lambda: w.all_gather([t[:25000] for t in x], y, 100000),
+                     lambda: w.send_recv([(0, 1, x[0], 200000, y[1], 200000)])):
+            with pytest.raises(HxcclError):
+                call()
+        graph.capture_end()
+    for count in (50000, 64):
+        for t in y:
+            t.zero_()
+        w.all_reduce(x, y, count, L.FLOAT32)
+        torch.cuda.synchronize()
+        assert all(bool((t[:count] == 3).all()) for t in y)
+    assert all(w.status(r) == (0, 0) for r in range(2))
