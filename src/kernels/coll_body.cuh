@@ -56,9 +56,9 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
       sh.piece_len[threadIdx.x] = a.send_bytes[j] > lo + by_mc ? min_sz(a.sub_bytes, a.send_bytes[j] - lo) - by_mc : 0;
     }
     if (kFold && a.push_scaled)
-      cta_pieces(sh, n - 1, a.sub_bytes, ScaleMover<T>{scalar});
-    else
-      cta_pieces(sh, n - 1, a.sub_bytes, CopyMover{});
+      cta_pieces(sh, n - 1, a.sub_bytes, ScaleMover<T>(scalar));
+    else  // a copy's source may be one block for every peer
+      cta_pieces(sh, n - 1, a.sub_bytes, CopyMover<kFold, false>{});
     __syncthreads();
     tm.lap(kTrIn);
     signal_all(w, kOffFlagsA, cta, e_step0 + step);
@@ -76,7 +76,7 @@ __device__ void xchg_body(const XchgArgs& a, int cta, int ncta, FoldShared& sh) 
         sh.piece_dst[threadIdx.x] = to;
         sh.piece_len[threadIdx.x] = a.recv_bytes[i] > lo && from != to ? min_sz(a.sub_bytes, a.recv_bytes[i] - lo) : 0;
       }
-      cta_pieces(sh, n, a.sub_bytes, CopyMover{});
+      cta_pieces(sh, n, a.sub_bytes, CopyMover<true, true>{});
     } else if (a.fold_bytes > lo) {
       const size_t len = min_sz(a.sub_bytes, a.fold_bytes - lo);
       __syncthreads();  // the previous fold is done with sh.src
@@ -159,12 +159,12 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
       sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
     if constexpr (kCast) {
-      cta_pieces(sh, np, a.sub_bytes, NarrowMover<T>{scalar, a.fold.premul != 0});
+      cta_pieces(sh, np, a.sub_bytes, NarrowMover<T>(scalar, a.fold.premul != 0));
     } else {
       if (a.fold.premul)
-        cta_pieces(sh, np, a.sub_bytes, ScaleMover<T>{scalar});
+        cta_pieces(sh, np, a.sub_bytes, ScaleMover<T>(scalar));
       else
-        cta_pieces(sh, np, a.sub_bytes, CopyMover{});
+        cta_pieces(sh, np, a.sub_bytes, CopyMover<true, false>{});
     }
     __syncthreads();
     tm.lap(kTrIn);
@@ -206,9 +206,9 @@ __device__ void twoshot_body(const TwoShotArgs& a, int cta, int ncta, FoldShared
       sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
     if constexpr (kCast)
-      cta_pieces(sh, np, a.sub_bytes, WidenMover<T>{});
+      cta_pieces(sh, np, a.sub_bytes, WidenMover<T>());
     else
-      cta_pieces(sh, np, a.sub_bytes, CopyMover{});
+      cta_pieces(sh, np, a.sub_bytes, CopyMover<true, true>{});
     __syncthreads();
     tm.lap(kTrOut);
   };

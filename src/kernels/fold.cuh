@@ -129,10 +129,10 @@ __device__ inline T fold_element(const FoldShared& sh, size_t e, size_t elem0, b
 // (16-byte aligned).
 template <typename T>
 __device__ __forceinline__ void fold_store(char* dst, bool dst_aligned, const FoldShared& sh, int nremote, unsigned v,
-                                           const Vec16<T>& out) {
+                                           const Vec16<T>& out, unsigned long long policy) {
   const size_t off = size_t(v) << 4;
   if (dst_aligned) {
-    st16(dst + off, out.raw);
+    st16_once_if(true, dst + off, out.raw, policy);
   } else {
 #pragma unroll
     for (int l = 0; l < int(16 / sizeof(T)); ++l) reinterpret_cast<T*>(dst + off)[l] = out.e[l];
@@ -159,6 +159,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
   using L = Lanes<T>;
   const FoldSpec& f = sh.spec;
   const int rank = sh.rank, n = kTree ? N : sh.n;
+  const unsigned long long policy = once_policy();  // every source is read for the last time
   constexpr int V = 16 / sizeof(T);
   const unsigned t = fresh_tid(), lane = t & 31u, warp = t >> 5, warps = blockDim.x >> 5;
   // the rank whose value comes k-th; its address is read from shared memory where it is needed (eight
@@ -178,7 +179,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
       const int idx = k < n ? rank_at(k) : rank;
       const char* p = sh.src[idx] + (size_t(v0) << 4) - (idx == rank ? shift : 0u);
 #pragma unroll
-      for (int u = 0; u < U; ++u) in[u][k].raw = ld16_if(u * 32 < left && k < n, p + u * 512);
+      for (int u = 0; u < U; ++u) in[u][k].raw = ld16_once_if(u * 32 < left && k < n, p + u * 512, policy);
     }
     if (shift) {  // cut the own vectors out of the two aligned ones they span
 #pragma unroll
@@ -260,7 +261,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 #pragma unroll
         for (int l = 0; l < V; ++l) out.e[l] = div_trunc(out.e[l], f.postdiv);
       }
-      fold_store<T>(dst, dst_aligned, sh, nremote, v, out);
+      fold_store<T>(dst, dst_aligned, sh, nremote, v, out, policy);
     }
   }
 }
@@ -277,8 +278,8 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 // Two to eight ranks keep every source of a vector in registers: kN is 2, 4 or 8 with kN/2 < n <= kN,
 // one kernel each (a kernel that carries all of them spills). What is left goes element by element with
 // the values in local memory: tails, trees, recursive doubling over other counts, and all of
-// kN = 0 (one rank, nine to sixteen ranks). Seven ranks, 28 MB fp32 average, on one B200: 677 us a call
-// when seven ranks took that general path, 243 us with the vector loop.
+// kN = 0 (one rank, nine to sixteen ranks). Seven ranks, 28 MB fp32 average, on one B200 (111 CTAs):
+// 677 us a call when seven ranks took that general path, 243 us with the vector loop.
 template <typename T, int kN>
 static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, int nremote, size_t nbytes, size_t elem0,
                                              bool premul, T scalar) {
@@ -294,7 +295,9 @@ static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, in
   };
   unsigned done = 0;  // elements that the vector loops cover
   if constexpr (kN >= 2) {
-    constexpr int U = 8 / kN;
+    // sixteen 16-byte loads in flight per thread; with eight, the ReduceScatter + AllGather of 14 MB on
+    // 8 ranks took 132 us instead of 125, 7 ranks' 28 MB fp32 average 195 instead of 188
+    constexpr int U = 16 / kN;
     const bool dst_aligned = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
     const bool ring = f.kind == kFoldLinear && f.ring, tree = f.kind == kFoldDoubling && n == kN;
     const unsigned nvec = f.kind == kFoldLinear || tree ? unsigned(nbytes >> 4) : 0;
@@ -389,15 +392,26 @@ __device__ __forceinline__ void cta_pieces(const FoldShared& sh, int np, size_t 
   }
 }
 
+// kOnceIn / kOnceOut: the source / the destination is not touched again soon
+template <bool kOnceIn, bool kOnceOut>
 struct CopyMover {
   using Elem = char;
   using Reg = uint4;
   static constexpr int kUnroll = 8;
+  unsigned long long policy;
+  __device__ __forceinline__ CopyMover() : policy(once_policy()) {}
   __device__ __forceinline__ bool fits(const char* dst, const char* src) const {
     return ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
   }
-  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const { return ld16_if(ok, src + (size_t(i) << 4)); }
-  __device__ __forceinline__ void store(bool ok, char* dst, unsigned i, uint4 v) const { st16_if(ok, dst + (size_t(i) << 4), v); }
+  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const {
+    const char* p = src + (size_t(i) << 4);
+    return kOnceIn ? ld16_once_if(ok, p, policy) : ld16_if(ok, p);
+  }
+  __device__ __forceinline__ void store(bool ok, char* dst, unsigned i, uint4 v) const {
+    char* p = dst + (size_t(i) << 4);
+    if (kOnceOut) st16_once_if(ok, p, v, policy);
+    else st16_if(ok, p, v);
+  }
   __device__ __forceinline__ void element(char* dst, const char* src, unsigned e) const { dst[e] = src[e]; }
   __device__ __forceinline__ void odd_pieces(const FoldShared& sh, int np) const {
     for (int j = 0; j < np; ++j) cta_copy(sh.piece_dst[j], sh.piece_src[j], sh.piece_len[j]);
@@ -408,12 +422,14 @@ template <typename T>
 struct ScaleMover {
   using Elem = T;
   using Reg = uint4;
-  static constexpr int kUnroll = 4;
+  static constexpr int kUnroll = 8;
   T scalar;
+  unsigned long long policy;
+  __device__ __forceinline__ explicit ScaleMover(T k) : scalar(k), policy(once_policy()) {}
   __device__ __forceinline__ bool fits(const char* dst, const char* src) const {
     return ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
   }
-  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const { return ld16_if(ok, src + (size_t(i) << 4)); }
+  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const { return ld16_once_if(ok, src + (size_t(i) << 4), policy); }
   __device__ __forceinline__ void store(bool ok, char* dst, unsigned i, uint4 v) const {
     Vec16<T> x;
     x.raw = v;
@@ -450,7 +466,7 @@ template <typename T>
 __device__ inline void cta_scale_copy(char* dst, const char* src, size_t nbytes, T scalar) {
   constexpr int V = 16 / sizeof(T);
   const unsigned t = threadIdx.x, nt = blockDim.x;
-  const ScaleMover<T> m{scalar};
+  const ScaleMover<T> m(scalar);
   const unsigned nvec = m.fits(dst, src) ? unsigned(nbytes >> 4) : 0;
   for (unsigned i = t; i < nvec; i += nt) m.store(true, dst, i, m.load(true, src, i));
   const unsigned total = unsigned(nbytes / sizeof(T));
@@ -495,12 +511,13 @@ struct NarrowMover {
   static constexpr int kUnroll = 4;
   T scalar;
   bool premul;
+  __device__ __forceinline__ NarrowMover(T k, bool p) : scalar(k), premul(p) {}
   __device__ __forceinline__ bool fits(const char* dst, const char* src) const {
     return ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
   }
   __device__ __forceinline__ Reg load(bool ok, const char* src, unsigned i) const {
     const char* p = src + (size_t(i) << 5);
-    return Reg{ld16_if(ok, p), ld16_if(ok, p + 16)};
+    return Reg{ld16_if(ok, p), ld16_if(ok, p + 16)};  // through L1: the two share sectors
   }
   __device__ __forceinline__ void store(bool ok, char* dst, unsigned i, const Reg& r) const {
     Vec16<T> x = narrow_lanes<T>(r.a, r.b);
@@ -520,10 +537,12 @@ struct WidenMover {
   using Elem = T;
   using Reg = uint4;
   static constexpr int kUnroll = 4;
+  unsigned long long policy;
+  __device__ __forceinline__ WidenMover() : policy(once_policy()) {}
   __device__ __forceinline__ bool fits(const char* dst, const char* src) const {
     return ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
   }
-  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const { return ld16_if(ok, src + (size_t(i) << 4)); }
+  __device__ __forceinline__ uint4 load(bool ok, const char* src, unsigned i) const { return ld16_once_if(ok, src + (size_t(i) << 4), policy); }
   __device__ __forceinline__ void store(bool ok, char* dst, unsigned i, uint4 v) const {
     Vec16<T> x;
     x.raw = v;

@@ -107,9 +107,9 @@ struct TwoShotRoleOps {
       sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
     if (a.fold.premul)
-      cta_pieces(sh, w.n - 1, a.sub_bytes, ScaleMover<T>{scalar});
+      cta_pieces(sh, w.n - 1, a.sub_bytes, ScaleMover<T>(scalar));
     else
-      cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover{});
+      cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover<true, false>{});
   }
   __device__ void combine(int k) {
     const WinView& w = a.w;
@@ -140,7 +140,7 @@ struct TwoShotRoleOps {
       sh.piece_dst[threadIdx.x] = a.recv + lo;
       sh.piece_len[threadIdx.x] = lo < a.bytes ? min_sz(a.sub_bytes, a.bytes - lo) : 0;
     }
-    cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover{});
+    cta_pieces(sh, w.n - 1, a.sub_bytes, CopyMover<true, true>{});
   }
 };
 
