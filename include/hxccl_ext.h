@@ -102,7 +102,9 @@ hxcclResult_t hxcclTestSeverPeer(hxcclComm_t comm, int peer);
 /* ---- a whole communicator on one GPU ------------------------------------------------------------ */
 typedef struct hxcclWorld* hxcclWorld_t;
 /* n ranks (1..16) on the current device, each with a window of window_mb MiB of staging.
- * wait_ms bounds every device-side wait. Calls on a stream that is being captured are refused. */
+ * wait_ms bounds every device-side wait. On two ranks or more, calls on a stream that is being
+ * captured are refused before anything is enqueued (a group of Sends and Recvs whose every transfer
+ * is from a rank to itself is plain copies and may be captured). */
 hxcclResult_t hxcclWorldCreate(hxcclWorld_t* world, int n, int window_mb, int wait_ms);
 hxcclResult_t hxcclWorldDestroy(hxcclWorld_t world);
 /* variant/exact/max_ctas as in hxcclCommTune */

@@ -67,6 +67,12 @@ hxcclResult_t rc_of(cudaError_t e) {
   g_last_error = cudaGetErrorString(e);
   return hxcclUnhandledCudaError;
 }
+
+// Asked by every call that has work for the lanes or the collective kernels, before anything is enqueued or
+// counted. A world of one rank waits for nobody: it takes the launches of a communicator, which may be captured.
+cudaError_t admit(const hxcclWorld* w, hxcclStream_t stream) {
+  return w->n > 1 ? refuse_capture(static_cast<cudaStream_t>(stream)) : cudaSuccess;
+}
 }  // namespace
 
 extern "C" {
@@ -163,6 +169,7 @@ hxcclResult_t hxcclWorldAllReduce(hxcclWorld_t w, const void* const* send, void*
   if (count == 0) return hxcclSuccess;
   if (order < 0) order = count * dtype_size(dt) < kDoublingMaxBytes ? kOrderDoubling : kOrderRing;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.allreduce(b.data(), count, dt, plan, order, static_cast<cudaStream_t>(stream)));
 }
 
@@ -175,6 +182,7 @@ hxcclResult_t hxcclWorldAllReduceCast(hxcclWorld_t w, const void* const* send, v
   if (count == 0) return hxcclSuccess;
   if (w->n < 2) return hxcclInvalidUsage;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.allreduce_cast(b.data(), count, wire_dt, plan, static_cast<cudaStream_t>(stream)));
 }
 
@@ -185,6 +193,7 @@ hxcclResult_t hxcclWorldReduceScatter(hxcclWorld_t w, const void* const* send, v
   if (!w || !make_plan(w->n, dt, op, scalar, &plan) || dtype_size(dt) == 0) return hxcclInvalidArgument;
   if (recvcount == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.reducescatter(b.data(), recvcount, dt, plan, static_cast<cudaStream_t>(stream)));
 }
 
@@ -196,6 +205,7 @@ hxcclResult_t hxcclWorldReduce(hxcclWorld_t w, const void* const* send, void* co
     return hxcclInvalidArgument;
   if (count == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.reduce(b.data(), count, dt, plan, root, static_cast<cudaStream_t>(stream)));
 }
 
@@ -204,6 +214,7 @@ hxcclResult_t hxcclWorldAllGather(hxcclWorld_t w, const void* const* send, void*
   if (!w) return hxcclInvalidArgument;
   if (bytes == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.allgather(b.data(), bytes, static_cast<cudaStream_t>(stream)));
 }
 hxcclResult_t hxcclWorldBroadcast(hxcclWorld_t w, const void* const* send, void* const* recv,
@@ -211,6 +222,7 @@ hxcclResult_t hxcclWorldBroadcast(hxcclWorld_t w, const void* const* send, void*
   if (!w || root < 0 || root >= w->n) return hxcclInvalidArgument;
   if (bytes == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.broadcast(b.data(), bytes, root, static_cast<cudaStream_t>(stream)));
 }
 hxcclResult_t hxcclWorldGather(hxcclWorld_t w, const void* const* send, void* const* recv,
@@ -218,6 +230,7 @@ hxcclResult_t hxcclWorldGather(hxcclWorld_t w, const void* const* send, void* co
   if (!w || root < 0 || root >= w->n) return hxcclInvalidArgument;
   if (bytes == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.gather(b.data(), bytes, root, static_cast<cudaStream_t>(stream)));
 }
 hxcclResult_t hxcclWorldScatter(hxcclWorld_t w, const void* const* send, void* const* recv,
@@ -225,6 +238,7 @@ hxcclResult_t hxcclWorldScatter(hxcclWorld_t w, const void* const* send, void* c
   if (!w || root < 0 || root >= w->n) return hxcclInvalidArgument;
   if (bytes == 0) return hxcclSuccess;
   auto b = bufs(w, send, recv);
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.scatter(b.data(), bytes, root, static_cast<cudaStream_t>(stream)));
 }
 
@@ -245,6 +259,7 @@ hxcclResult_t hxcclWorldAllToAllv(hxcclWorld_t w, const void* const* send, void*
   for (int r = 0; r < n; ++r)
     v[r] = RankV{static_cast<const char*>(send[r]), bytes + size_t(r) * n, soff + size_t(r) * n,
                  static_cast<char*>(recv[r]), rbytes.data() + size_t(r) * n, roff + size_t(r) * n};
+  if (cudaError_t e = admit(w, stream)) return rc_of(e);
   return rc_of(w->eng.alltoallv(v.data(), max_pair, static_cast<cudaStream_t>(stream)));
 }
 
@@ -253,11 +268,15 @@ hxcclResult_t hxcclWorldSendRecv(hxcclWorld_t w, int nops, const int* from, cons
                                  const size_t* rbytes, hxcclStream_t stream) {
   if (!w || nops < 0) return hxcclInvalidArgument;
   std::vector<RankP2p> per(w->n);
+  bool lanes = false;
   for (int k = 0; k < nops; ++k) {
     if (from[k] < 0 || from[k] >= w->n || to[k] < 0 || to[k] >= w->n) return hxcclInvalidArgument;
+    lanes = lanes || from[k] != to[k];
     per[from[k]].ops.push_back(P2pOp{true, to[k], const_cast<void*>(src[k]), sbytes[k]});
     per[to[k]].ops.push_back(P2pOp{false, from[k], dst[k], rbytes[k]});
   }
+  // transfers of a rank to itself are plain copies, which may be captured
+  if (cudaError_t e = lanes ? admit(w, stream) : cudaSuccess) return rc_of(e);
   return rc_of(w->eng.p2p(per.data(), static_cast<cudaStream_t>(stream)));
 }
 

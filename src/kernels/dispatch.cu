@@ -134,7 +134,6 @@ static cudaError_t launch_p2p_world(const P2pArgs* args, LaunchShape s, cudaStre
   P2pWorldArgs<kLanes, kOps> a;
   static_assert(sizeof a <= 32764, "kernel parameters");
   if (s.world > kMaxRanks) return cudaErrorInvalidValue;
-  if (cudaError_t e = refuse_capture(st)) return e;
   int lane = 0, op = 0;
   a.workers_per_cta = args[0].workers_per_cta;
   for (int r = 0; r < s.world; ++r) {

@@ -86,19 +86,10 @@ __global__ void __launch_bounds__(256, 1) k_ll_world(const __grid_constant__ Wor
   ll_body<T, kN>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);
 }
 
-// A world's call is refused on a stream that is being captured: its epochs are part of the launch,
-// and a replay would meet flags that are already up.
-inline cudaError_t refuse_capture(cudaStream_t st) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  const cudaError_t e = cudaStreamIsCapturing(st, &status);
-  return e == cudaSuccess && status != cudaStreamCaptureStatusNone ? cudaErrorStreamCaptureUnsupported : e;
-}
-
 template <int kN = 0, typename Args>
 cudaError_t launch_world(const void* kernel, const Args* args, LaunchShape s, cudaStream_t st) {
   static_assert(sizeof(WorldArgs<Args, kN>) <= 32764, "kernel parameters");
   if (s.world > (kN ? kN : kMaxRanks)) return cudaErrorInvalidValue;
-  if (cudaError_t e = refuse_capture(st)) return e;
   WorldArgs<Args, kN> all;  // blocks of ranks that do not exist stay unset: no CTA reads them
   memcpy(all.rank, args, sizeof(Args) * size_t(s.world));
   void* params[] = {&all};

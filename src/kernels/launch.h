@@ -16,6 +16,15 @@ struct LaunchShape {
   int world;  // 0 = production (one rank per GPU)
 };
 
+// An error when `st` is being captured. The epochs of a launch over several ranks in one grid are part of
+// its parameters, and a replay would meet flags that are already up, so whoever launches that form asks
+// here before it enqueues or counts anything.
+inline cudaError_t refuse_capture(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(st, &status);
+  return e == cudaSuccess && status != cudaStreamCaptureStatusNone ? cudaErrorStreamCaptureUnsupported : e;
+}
+
 cudaError_t launch_xchg_copy(const XchgArgs* args, LaunchShape s, cudaStream_t st);
 cudaError_t launch_xchg_fold(int dt, const XchgArgs* args, LaunchShape s, cudaStream_t st);
 cudaError_t launch_twoshot(int dt, const TwoShotArgs* args, LaunchShape s, cudaStream_t st);

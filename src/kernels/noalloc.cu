@@ -68,6 +68,7 @@ extern "C" hxcclResult_t hxcclAllReduceNoAlloc(int nranks, const void* const* se
   if (dev < 0 || dev >= kMaxDevices) return fail(hxcclInvalidArgument, "device ordinal out of range");
   PerDevice& pd = g_dev[dev];
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if ((e = refuse_capture(st)) != cudaSuccess) return fail(hxcclUnhandledCudaError, "the stream is being captured", e);
   {  // The array's device address, with this device current. The first call on a device is
      // the set-up; later calls repeat the (cheap) look-up instead of trusting a cached pointer,
      // which a cudaDeviceReset or another context on the same ordinal would leave stale. A

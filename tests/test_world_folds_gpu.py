@@ -155,3 +155,50 @@ def test_a_world_refuses_a_capturing_stream(worlds):
         torch.cuda.synchronize()
         assert all(bool((t[:count] == 3).all()) for t in y)
     assert all(w.status(r) == (0, 0) for r in range(2))
+
+
+def test_capture_is_refused_before_anything_is_recorded(worlds):
+    """A refused call records nothing and counts nothing; what waits for nobody (transfers of a rank to
+    itself, a world of one rank) is captured and replays."""
+    from hxccl_b200.comm import HxcclError
+
+    w, single = worlds(2), worlds(1)
+    x = [torch.zeros(5000, device="cuda") for _ in range(2)]
+    y = [torch.zeros_like(t) for t in x]
+    z, marker = torch.zeros_like(x[0]), torch.zeros_like(x[0])
+    nb = x[0].nbytes
+    to_self, across = [(0, 0, x[0], nb, y[0], nb)], [(0, 1, x[0], nb, y[1], nb)]
+
+    def one_rank():
+        single.all_reduce([x[1]], [y[1]], 5000, L.FLOAT32)
+        single.reduce_scatter([x[1]], [z], 5000, L.FLOAT32, op=L.AVG)
+
+    one_rank()  # kernels are loaded before the capture
+    torch.cuda.synchronize()
+    refused, graph = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        before = w.info()
+        refused.capture_begin()
+        marker.fill_(1)
+        with pytest.raises(HxcclError):
+            w.send_recv(to_self + across)
+        with pytest.raises(HxcclError):
+            w.all_reduce(x, y, 5000, L.FLOAT32)
+        refused.capture_end()
+        assert w.info() == before
+        graph.capture_begin()
+        w.send_recv(to_self)
+        one_rank()
+        graph.capture_end()
+    for k in (1.0, 2.0):
+        for t in x:
+            t.fill_(k)
+        for t in y:
+            t.zero_()
+        refused.replay()
+        torch.cuda.synchronize()
+        assert bool(marker.all()) and not any(bool(t.any()) for t in y)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(bool((t == k).all()) for t in (y[0], y[1], z))
+    assert single.status(0) == (0, 0)
