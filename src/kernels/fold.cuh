@@ -275,11 +275,12 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 // The ring order changes its starting rank from ring block to ring block. A share is usually inside
 // one block, so the block is looked up once per stretch of vectors between two block ends, not per
 // vector; a vector that straddles two blocks goes element by element, like the tail.
-// Two to eight ranks keep every source of a vector in registers: kN is 2, 4 or 8 with kN/2 < n <= kN,
-// one kernel each (a kernel that carries all of them spills). What is left goes element by element with
-// the values in local memory: tails, trees, recursive doubling over other counts, and all of
-// kN = 0 (one rank, nine to sixteen ranks). Seven ranks, 28 MB fp32 average, on one B200 (111 CTAs):
-// 677 us a call when seven ranks took that general path, 243 us with the vector loop.
+// The linear orders keep every source of a vector in registers: kN is 2, 4 or 8 with kN/2 < n <= kN,
+// one kernel each (a kernel that carries all of them spills), and 0 for one rank and for nine to sixteen,
+// whose loop is sixteen wide. What is left goes element by element with the values in local memory:
+// tails, trees, recursive doubling over other counts. One B200, us a call: 7 ranks, 28 MB fp32 average, 677 by
+// that general path and 243 by vectors (111 CTAs); 9 ranks, 16 MiB e4m3, 748 and 165; 12 ranks, 16 MiB
+// fp32, 355 and 201.
 template <typename T, int kN>
 static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, int nremote, size_t nbytes, size_t elem0,
                                              bool premul, T scalar) {
@@ -293,43 +294,47 @@ static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, in
     reinterpret_cast<T*>(dst)[e] = r;
     for (int q = 0; q < nremote; ++q) reinterpret_cast<T*>(sh.remote[q])[e] = r;
   };
-  unsigned done = 0;  // elements that the vector loops cover
-  if constexpr (kN >= 2) {
-    // sixteen 16-byte loads in flight per thread; with eight, the ReduceScatter + AllGather of 14 MB on
-    // 8 ranks took 132 us instead of 125, 7 ranks' 28 MB fp32 average 195 instead of 188
-    constexpr int U = 16 / kN;
-    const bool dst_aligned = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
-    const bool ring = f.kind == kFoldLinear && f.ring, tree = f.kind == kFoldDoubling && n == kN;
-    const unsigned nvec = f.kind == kFoldLinear || tree ? unsigned(nbytes >> 4) : 0;
-    for (unsigned v = 0; v < nvec;) {
-      unsigned v_hi = nvec;  // whole vectors up to here take the sources in the same sequence
-      int first = f.start;
-      if (ring) {
-        const int block = ring_block_of(sh, elem0 + size_t(v) * V, n);
-        const size_t left = (block + 1 < n ? sh.bound[block + 1] : ~0ull) - elem0;  // elements up to the block's end
-        if (left / V < nvec) v_hi = unsigned(left / V);
-        first = (f.start + block) % n;
-      }
-      if (v_hi == v) {  // the vector straddles the end of the block
-        if (t < unsigned(V)) element(v * V + t);
-        ++v;
-        continue;
-      }
+  constexpr int N = kN ? kN : kMaxRanks;
+  // sixteen 16-byte loads in flight per thread; with eight, the ReduceScatter + AllGather of 14 MB on
+  // 8 ranks took 132 us instead of 125, 7 ranks' 28 MB fp32 average 195 instead of 188
+  constexpr int U = 16 / N;
+  const bool dst_aligned = (reinterpret_cast<uintptr_t>(dst) & 15u) == 0;
+  const bool ring = f.kind == kFoldLinear && f.ring, tree = f.kind == kFoldDoubling && n == kN;
+  // below four elements per thread the sixteen-wide loop leaves most threads idle (9 ranks, 1 MiB fp32 max:
+  // 26.9 us a call, by elements 24.5)
+  const bool vectors = (f.kind == kFoldLinear && (kN || total > 4 * nt)) || tree;
+  const unsigned nvec = vectors ? unsigned(nbytes >> 4) : 0;
+  for (unsigned v = 0; v < nvec;) {
+    unsigned v_hi = nvec;  // whole vectors up to here take the sources in the same sequence
+    int first = f.start;
+    if (ring) {
+      const int block = ring_block_of(sh, elem0 + size_t(v) * V, n);
+      const size_t left = (block + 1 < n ? sh.bound[block + 1] : ~0ull) - elem0;  // elements up to the block's end
+      if (left / V < nvec) v_hi = unsigned(left / V);
+      first = (f.start + block) % n;
+    }
+    if (v_hi == v) {  // the vector straddles the end of the block
+      if (t < unsigned(V)) element(v * V + t);
+      ++v;
+      continue;
+    }
+    if constexpr (kN >= 2) {
       if (tree) {
         if (f.op == kSum)
-          fold_vectors<T, kN, 1, kSum, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
+          fold_vectors<T, N, 1, kSum, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
         else
-          fold_vectors<T, kN, 1, -1, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
-      } else if (f.op == kSum) {
-        fold_vectors<T, kN, U, kSum, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
-      } else {
-        fold_vectors<T, kN, 1, -1, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
+          fold_vectors<T, N, 1, -1, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
+        v = v_hi;
+        continue;
       }
-      v = v_hi;
     }
-    done = nvec * V;
+    if (f.op == kSum)
+      fold_vectors<T, N, U, kSum, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
+    else
+      fold_vectors<T, N, 1, -1, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
+    v = v_hi;
   }
-  for (unsigned e = done + t; e < total; e += nt) element(e);
+  for (unsigned e = nvec * V + t; e < total; e += nt) element(e);
 }
 
 // ---- moving the pieces of a step ---------------------------------------------------------------------

@@ -202,3 +202,37 @@ def test_capture_is_refused_before_anything_is_recorded(worlds):
         torch.cuda.synchronize()
         assert all(bool((t == k).all()) for t in (y[0], y[1], z))
     assert single.status(0) == (0, 0)
+
+
+@pytest.mark.parametrize("n", [3, 6, 9, 16])
+def test_orders_without_a_loop_of_their_own(worlds, n):
+    """Nine ranks and more, recursive doubling over 3 and 6 ranks, binomial trees: shares of whole vectors
+    per thread and shares below that, block ends inside vectors, aligned and odd buffers, in place."""
+    w = worlds(n)
+    rng = np.random.default_rng(100 + n)
+    for dt, op in ((L.FLOAT32, L.SUM), (L.BFLOAT16, L.AVG), (L.FLOAT8E4M3, L.SUM), (L.INT32, L.AVG), (L.INT8, L.MAX)):
+        es = L.DTYPE_SIZE[dt]
+        for count in (2999, 300007):
+            xs = [rng.integers(0, 256, count * es, dtype=np.uint8).view(oracle.raw_dtype(dt)) for _ in range(n)]
+            for variant, order in ((1, 0), (1, 1), (2, 0)):
+                want = oracle.allreduce(xs, dt, op, order=order)
+                w.tune(variant=variant, exact=True)
+                for shift in (0, es):
+                    buf = [dev(x, shift) for x in xs]
+                    w.all_reduce(buf, buf, count, dt, op=op, order=order)
+                    torch.cuda.synchronize()
+                    for r in range(n):
+                        assert np.array_equal(back(buf[r], dt), want[r]), (n, dt, count, variant, order, shift, r)
+            per = count // n
+            send = [dev(x[:per * n], es) for x in xs]
+            recv = [torch.zeros(per * es, dtype=torch.uint8, device="cuda") for _ in range(n)]
+            w.reduce_scatter(send, recv, per, dt, op=op)
+            out = [dev(np.zeros_like(xs[0])) if r == n - 1 else None for r in range(n)]
+            w.reduce([dev(x) for x in xs], out, count, dt, n - 1, op=op)
+            torch.cuda.synchronize()
+            want = oracle.reducescatter([x[:per * n] for x in xs], dt, op)
+            for r in range(n):
+                assert np.array_equal(back(recv[r], dt), want[r]), ("rs", n, dt, count, r)
+            assert np.array_equal(back(out[n - 1], dt), oracle.reduce(xs, dt, op, n - 1)), ("reduce", n, dt, count)
+    w.tune(variant=0, exact=True)
+    assert all(w.status(r) == (0, 0) for r in range(n))
