@@ -28,6 +28,15 @@ Tuning Engine::lean(const Tuning& t) const {
   return out;
 }
 
+bool Engine::ring_in_vectors(const RankBufs* b, size_t count, size_t es) const {
+  const size_t base = count / size_t(n()), extra = count % size_t(n());
+  for (size_t k = 1; k < size_t(n()); ++k)
+    if ((k * base + std::min(k, extra)) * es % 16) return false;
+  for (size_t r = 0; r < views.size(); ++r)
+    if ((reinterpret_cast<uintptr_t>(b[r].send) | reinterpret_cast<uintptr_t>(b[r].recv)) & 15u) return false;
+  return true;
+}
+
 cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpPlan& plan,
                               int order, cudaStream_t st) {
   const size_t bytes = count * dtype_size(dt);
@@ -47,6 +56,11 @@ cudaError_t Engine::allreduce(const RankBufs* b, size_t count, int dt, const OpP
   }
   const TuneRow* row = nullptr;
   int var = choose_variant(bytes, dt, plan, n(), tune, forced_variant, &row);
+  // The ring moves vectors only where all its blocks start on 16 bytes, and one element per thread and load
+  // elsewhere; the two-shot's slices always do. A world sees the buffers of every rank, so it can choose
+  // by that (one B200, us a call, ring and two-shot: 7 ranks, 64 MiB - 4 fp32 1047 and 437, bf16 1870 and 437,
+  // e4m3 3537 and 465; 3 ranks, 200 MiB - 4 fp32 1198 and 509).
+  if (world() && var == kVarRing && forced_variant == kVarAuto && !row && !ring_in_vectors(b, count, dtype_size(dt))) var = kVarTwoShot;
   const Tuning tune = with_row(this->tune, row, var);  // the row's launch shape, for this call only
   // recursive doubling gives every rank its own operand order; only the variant in which each
   // rank folds for itself can replay that

@@ -65,6 +65,8 @@ class Engine {
   cudaError_t p2p(const RankP2p* ops, cudaStream_t st);
 
  private:
+  // every block of a ring AllReduce over these buffers starts on a 16-byte boundary, on every rank
+  bool ring_in_vectors(const RankBufs* b, size_t count, size_t es) const;
   LaunchShape shape(const Geometry& g) const;
   uint64_t ll_era_ = 0;  // upper half of the epoch the line region was last cleared for
 };

@@ -115,16 +115,19 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
   w->eng.world_lean = true;
   w->eng.tune.threads = 512;  // one CTA per SM: the budget above counts on it
   w->eng.tune.roles_min_ranks = 2;
-  // Where the lines lie when all ranks share one GPU (one B200, us a call, fp32 sum):
+  // Where the lines lie when all ranks share one GPU (one B200, us a call, fp32 sum unless said otherwise):
   //   lines up to 64 KiB      8 ranks, 40 KiB bf16: lines 16.3, one-shot 17.1; 8 ranks, 256 KiB: 28.1 and 16.9
   //   4 KiB grain             8 ranks, 512 KiB two-shot: 17.2, with 16 KiB 22.4; 1 MiB 19.3 and 23.1
-  //   ring from 48 MiB        2 ranks, 64 MiB: ring 93, two-shot 119; 16 MiB: 40 and 32; 8 ranks, 64 MiB: 425 and
-  //                           511, 16 MiB: 144 and 133. Never the role pipeline: 16 MiB on 4 ranks 152, two-shot 86
-  //   hops of 64 KiB on two ranks (256 MiB: 289; 128 KiB: 311; 512 KiB: 366), 128 KiB on more (4 ranks,
-  //                           64 MiB: 206; 64 KiB: 220): the slots of all CTAs then stay in L2
+  //   ring from 40 MiB on two ranks (32 MiB: ring 53, two-shot 50; 40 MiB: 71 and 95), from 56 MiB on more, for 4-, 2-
+  //                           and 1-byte types (4 ranks, 48 MiB: 189 and 171; 56 MiB: 194 and 200; 8 ranks:
+  //                           400 and 381, 409 and 440; 12 ranks: 623 and 606, 646 and 703). Where the last
+  //                           round is nearly empty it loses up to 6 % again (8 ranks, 80 MiB e4m3: 695 and 661).
+  //                           Never the role pipeline: 16 MiB on 4 ranks 152, two-shot 86
+  //   hops of 64 KiB on two ranks (256 MiB: 289; 128 KiB: 311; 512 KiB: 366): the slots of all CTAs, 39 MB, then
+  //                           stay in L2. 128 KiB on more (4 ranks, 64 MiB: 206; 64 KiB: 220)
   w->eng.tune.ll_max = 64 * 1024;
   w->eng.tune.grain = 4 * 1024;
-  w->eng.tune.ring_min = 48u << 20;
+  w->eng.tune.ring_min = size_t(n == 2 ? 40 : 56) << 20;
   w->eng.tune.roles_min = ~size_t(0);
   w->eng.tune.ring_sub = (n == 2 ? 64 : 128) * 1024;
   *out = w;

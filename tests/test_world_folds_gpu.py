@@ -236,3 +236,27 @@ def test_orders_without_a_loop_of_their_own(worlds, n):
             assert np.array_equal(back(out[n - 1], dt), oracle.reduce(xs, dt, op, n - 1)), ("reduce", n, dt, count)
     w.tune(variant=0, exact=True)
     assert all(w.status(r) == (0, 0) for r in range(n))
+
+
+def test_a_world_takes_the_ring_where_its_blocks_are_aligned(worlds):
+    """Blocks or buffers off the 16-byte grid go to the two-shot, unless the ring is asked for."""
+    n, count = 3, 3 << 17
+    w = worlds(n)
+    rng = np.random.default_rng(5)
+    w.knob("ring_min", 1 << 20)
+    try:
+        for odd, shifts, forced, variant in ((0, (0, 0, 0), 0, 6), (1, (0, 0, 0), 0, 2), (2, (0, 0, 0), 0, 2), (0, (0, 4, 0), 0, 2),
+                                             (1, (4, 0, 4), 6, 6)):
+            w.tune(variant=forced, exact=True)
+            xs = [rng.integers(0, 256, (count + odd) * 4, dtype=np.uint8).view(np.uint32) for _ in range(n)]
+            send, recv = [dev(x) for x in xs], [dev(np.zeros_like(x), s) for x, s in zip(xs, shifts)]
+            w.all_reduce(send, recv, count + odd, L.FLOAT32)
+            torch.cuda.synchronize()
+            assert w.info()["variant"] == variant, (odd, shifts, forced)
+            want = oracle.allreduce(xs, L.FLOAT32, L.SUM)
+            for r in range(n):
+                assert np.array_equal(back(recv[r], L.FLOAT32), want[r]), (odd, shifts, forced, r)
+    finally:
+        w.knob("ring_min", 56 << 20)
+        w.tune(variant=0, exact=True)
+    assert all(w.status(r) == (0, 0) for r in range(n))
