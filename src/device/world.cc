@@ -116,7 +116,10 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
   w->eng.tune.threads = 512;  // one CTA per SM: the budget above counts on it
   w->eng.tune.roles_min_ranks = 2;
   // Where the lines lie when all ranks share one GPU (one B200, us a call, fp32 sum unless said otherwise):
-  //   lines up to 64 KiB      8 ranks, 40 KiB bf16: lines 16.3, one-shot 17.1; 8 ranks, 256 KiB: 28.1 and 16.9
+  //   lines up to 64 KiB      2 ranks, 62 KiB: lines 10.6, one-shot 12.1; 8 ranks: 15.5 and 16.4. Rank counts whose
+  //                           lines kernel is the general one only as long as every thread has one line:
+  //                           7 ranks, e4m3, 42 KiB: 21.6 and 30.2, 46 KiB: 37.7 and 33.1; 12 ranks, 20 KiB: 19.2
+  //                           and 20.2, 28 KiB: 29.9 and 21.7
   //   4 KiB grain             8 ranks, 512 KiB two-shot: 17.2, with 16 KiB 22.4; 1 MiB 19.3 and 23.1
   //   ring from 40 MiB on two ranks (32 MiB: ring 53, two-shot 50; 40 MiB: 71 and 95), from 56 MiB on more, for 4-, 2-
   //                           and 1-byte types (4 ranks, 48 MiB: 189 and 171; 56 MiB: 194 and 200; 8 ranks:
@@ -125,7 +128,8 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
   //                           Never the role pipeline: 16 MiB on 4 ranks 152, two-shot 86
   //   hops of 64 KiB on two ranks (256 MiB: 289; 128 KiB: 311; 512 KiB: 366): the slots of all CTAs, 39 MB, then
   //                           stay in L2. 128 KiB on more (4 ranks, 64 MiB: 206; 64 KiB: 220)
-  w->eng.tune.ll_max = 64 * 1024;
+  const bool own_lines_kernel = n == 2 || n == 4 || n == 8;
+  w->eng.tune.ll_max = std::min<size_t>(64 * 1024, own_lines_kernel ? ~size_t(0) : size_t(w->eng.tune.max_ctas) * 256 * 8);
   w->eng.tune.grain = 4 * 1024;
   w->eng.tune.ring_min = size_t(n == 2 ? 40 : 56) << 20;
   w->eng.tune.roles_min = ~size_t(0);

@@ -260,3 +260,21 @@ def test_a_world_takes_the_ring_where_its_blocks_are_aligned(worlds):
         w.knob("ring_min", 56 << 20)
         w.tune(variant=0, exact=True)
     assert all(w.status(r) == (0, 0) for r in range(n))
+
+
+@pytest.mark.parametrize("n,kib,lines", [(7, 40, True), (7, 46, False), (8, 62, True), (12, 23, True), (12, 27, False)])
+def test_lines_end_where_a_thread_would_have_two(worlds, n, kib, lines):
+    """The general lines kernel (any count but 2, 4 and 8) is left before its threads take a second line."""
+    w = worlds(n)
+    w.tune(variant=0, exact=True)
+    count = kib * 256 - 1
+    rng = np.random.default_rng(n)
+    xs = [rng.integers(0, 256, count * 4, dtype=np.uint8).view(np.uint32) for _ in range(n)]
+    buf = [dev(x) for x in xs]
+    w.all_reduce(buf, buf, count, L.FLOAT32)
+    torch.cuda.synchronize()
+    assert (w.info()["variant"] == 7) == lines
+    want = oracle.allreduce(xs, L.FLOAT32, L.SUM)
+    for r in range(n):
+        assert np.array_equal(back(buf[r], L.FLOAT32), want[r]), (n, kib, r)
+    assert all(w.status(r) == (0, 0) for r in range(n))
