@@ -202,7 +202,10 @@ cudaError_t launch_reduce_t(void* dst, const void* src, size_t count, int op, cu
 template <typename T>
 cudaError_t launch_scale_t(void* dst, const void* src, size_t count, unsigned long long bits,
                            const void* scalar_ptr, cudaStream_t st) {
-  k_scale<T><<<elementwise_grid(count, 4 * 16 / sizeof(T)), 256, 0, st>>>(
+  // off the 16-byte grid the kernel goes element by element: a thread for each, not for each run of vectors
+  // (16 KiB e4m3 at an odd address, in place: 8.3 us a call on one B200, 23.0 with the vectors' grid)
+  const bool vectors = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
+  k_scale<T><<<elementwise_grid(count, vectors ? 4 * 16 / sizeof(T) : 1), 256, 0, st>>>(
       static_cast<T*>(dst), static_cast<const T*>(src), count, bits, scalar_ptr);
   return cudaGetLastError();
 }

@@ -2,6 +2,8 @@
 codes and every 16-bit code against awkward partners, every rank count that has a loop of its own,
 blocks that end inside a vector, buffers at any element offset. Compared bit for bit with the host
 schedules (hxccl_b200.ops.oracle)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -104,28 +106,46 @@ def test_rank_counts_block_ends_and_offsets(worlds, n):
     assert all(w.status(r) == (0, 0) for r in range(n))
 
 
-@pytest.mark.parametrize("dt", [L.FLOAT32, L.BFLOAT16, L.FLOAT8E5M2, L.INT64])
+def scalars(dt):
+    """1/8 is exact in every type; 3 overflows large values and rounds the others"""
+    if dt <= L.UINT64:
+        return [np.array([v & ((1 << (8 * L.DTYPE_SIZE[dt])) - 1)], dtype=oracle.raw_dtype(dt)) for v in (3, -5)]
+    if dt in (L.FLOAT32, L.FLOAT64):
+        return [np.array([v], dtype=np.float32 if dt == L.FLOAT32 else np.float64).view(oracle.raw_dtype(dt)) for v in (0.125, -3.3)]
+    return [np.array([L.lib().hxcclHostEncode(dt, C.c_float(v))], dtype=oracle.raw_dtype(dt)) for v in (0.125, -3.0)]
+
+
+@pytest.mark.parametrize("dt", [L.FLOAT32, L.FLOAT64, L.FLOAT16, L.BFLOAT16, L.FLOAT8E4M3, L.FLOAT8E5M2, L.INT64, L.INT8])
 def test_one_rank_scales(dt):
-    """Avg and PreMulSum over one rank: one scaling pass, any alignment, in place and out of place."""
+    """Avg and PreMulSum over one rank against the host rules: random codes (NaN and overflow among them),
+    any alignment, in place and out of place, the scalar given by value and in device memory written just
+    before on the same stream."""
     import hxccl_b200 as hx
+    from hxccl_b200.ops.world import World
 
     torch.zeros(1, device="cuda")
     comm = hx.Communicator.init_rank(hx.get_unique_id(), 1, 0)
-    from hxccl_b200.ops.world import World
-
     rng = np.random.default_rng(dt)
-    tdt = {L.FLOAT32: torch.float32, L.BFLOAT16: torch.bfloat16, L.FLOAT8E5M2: torch.float8_e5m2, L.INT64: torch.int64}[dt]
     es = L.DTYPE_SIZE[dt]
-    with World(1, window_mb=4, wait_ms=20000) as w:  # the kernels' own one-rank form
+    with World(1, window_mb=4, wait_ms=20000) as w:
         for count in (1, 15, 128, 129, 300007):
             x = rng.integers(0, 256, count * es, dtype=np.uint8).view(oracle.raw_dtype(dt))
             for shift in (0, es):
-                a, out, ref = dev(x, shift), dev(np.zeros_like(x), shift), dev(np.zeros_like(x))
-                comm.all_reduce(a.view(tdt), out.view(tdt), op=hx.AVG)
-                w.all_reduce([a], [ref], count, dt, op=L.AVG)
-                comm.all_reduce(a.view(tdt), a.view(tdt), op=hx.AVG)
+                a, out = dev(x, shift), dev(np.zeros_like(x), shift)
+                comm.all_reduce(a, out, op=hx.AVG, count=count, dtype=dt)
                 torch.cuda.synchronize()
-                assert torch.equal(out, ref) and torch.equal(a, ref), (dt, count, shift)
+                assert np.array_equal(back(out, dt), oracle.allreduce([x], dt, L.AVG)[0]), (dt, count, shift)
+                for k in scalars(dt):
+                    want = oracle.allreduce([x], dt, L.SUM, scalar=k)[0]
+                    b, on_device = dev(x, shift), dev(np.zeros_like(k))
+                    w.all_reduce([a], [out], count, dt, scalar=k)
+                    op = comm.create_premul_sum(on_device, dtype=dt, residence=L.SCALAR_DEVICE)
+                    on_device.copy_(dev(k))
+                    comm.all_reduce(b, b, op=op, count=count, dtype=dt)
+                    torch.cuda.synchronize()
+                    comm.destroy_op(op)
+                    assert np.array_equal(back(out, dt), want), ("by value", dt, count, shift, k)
+                    assert np.array_equal(back(b, dt), want), ("in device memory", dt, count, shift, k)
     comm.destroy()
 
 
