@@ -149,6 +149,51 @@ def test_one_rank_scales(dt):
     comm.destroy()
 
 
+@pytest.mark.parametrize("n", [2, 3, 8])
+def test_narrow_wire_type_at_any_alignment(worlds, n):
+    """hxcclAllReduceCast on fp32 buffers off the 16-byte grid, which move element by element."""
+    w = worlds(n)
+    w.tune(variant=0, exact=True)
+    for wire, tdt in ((L.BFLOAT16, torch.bfloat16), (L.FLOAT16, torch.float16)):
+        for op, count in ((L.AVG, 70001), (L.SUM, 32771)):
+            g = torch.Generator().manual_seed(count + wire)
+            xs = [(torch.randn(count, generator=g) * 3).float() for _ in range(n)]
+            want = oracle.allreduce([x.to(tdt).view(torch.uint16).numpy().copy() for x in xs], wire, op, order=0)
+            want32 = [torch.from_numpy(v.copy()).view(tdt).float().numpy() for v in want]
+            for from_shift, to_shift in ((4, 4), (8, 0), (0, 12)):
+                send = [dev(x.numpy(), from_shift) for x in xs]
+                recv = [dev(np.zeros(count, dtype=np.float32), to_shift) for _ in range(n)]
+                w.all_reduce_cast(send, recv, count, wire, op=op)
+                w.all_reduce_cast(send, send, count, wire, op=op)  # in place
+                torch.cuda.synchronize()
+                for r in range(n):
+                    for got in (recv[r], send[r]):
+                        assert np.array_equal(got.cpu().numpy(), want32[r].view(np.uint8)), (n, wire, op, from_shift, to_shift, r)
+    assert all(w.status(r) == (0, 0) for r in range(n))
+
+
+@pytest.mark.parametrize("n,each", [(2, 20), (8, 3), (12, 5)])
+def test_full_send_recv_groups(worlds, n, each):
+    """Groups over all pairs of ranks: more operations than a lane takes at once (2 ranks), than the small
+    parameter block holds (8 ranks: 112 lanes, 336 operations), than any launch carries (12 ranks: 1320
+    operations). Sizes differ within a lane, so an operation out of order would not match its buffer."""
+    w = worlds(n)
+    rng = np.random.default_rng(n)
+    moves = []
+    for k in range(each):
+        for r in range(n):
+            for j in range(n):
+                if r != j:
+                    size = int(rng.integers(0, 6000))
+                    moves.append((r, j, torch.from_numpy(rng.integers(0, 256, size + 1, dtype=np.uint8)).cuda(), size,
+                                  torch.full((size + 1,), 0xEE, dtype=torch.uint8, device="cuda"), size))
+    w.send_recv(moves)
+    torch.cuda.synchronize()
+    for r, j, src, size, dst, _ in moves:
+        assert torch.equal(dst[:size], src[:size]) and int(dst[size]) == 0xEE, (n, r, j, size)
+    assert all(w.status(r) == (0, 0) for r in range(n))
+
+
 def test_a_world_refuses_a_capturing_stream(worlds):
     """The epochs of a world's launch are baked into its parameters, so a replay would be wrong: calls on
     a capturing stream fail, and the world works on afterwards."""
