@@ -126,13 +126,14 @@ __device__ inline T fold_element(const FoldShared& sh, size_t e, size_t elem0, b
   return f.postdiv ? div_trunc(r, f.postdiv) : r;
 }
 // dst may have any alignment that its element type has; the remote destinations are window slots
-// (16-byte aligned).
-template <typename T>
+// (16-byte aligned). kDstOnce: dst is not read again soon (a caller's buffer).
+template <typename T, bool kDstOnce>
 __device__ __forceinline__ void fold_store(char* dst, bool dst_aligned, const FoldShared& sh, int nremote, unsigned v,
                                            const Vec16<T>& out, unsigned long long policy) {
   const size_t off = size_t(v) << 4;
   if (dst_aligned) {
-    st16_once_if(true, dst + off, out.raw, policy);
+    if (kDstOnce) st16_once_if(true, dst + off, out.raw, policy);
+    else st16(dst + off, out.raw);
   } else {
 #pragma unroll
     for (int l = 0; l < int(16 / sizeof(T)); ++l) reinterpret_cast<T*>(dst + off)[l] = out.e[l];
@@ -153,7 +154,7 @@ __device__ __forceinline__ void fold_store(char* dst, bool dst_aligned, const Fo
 // the level before on the left and its partner's on the right, and the partner's is formed the same way
 // from the partner's side. Only N - 1 of the N log N combinations of the butterfly feed rank r's
 // result, and with the sources in the order r ^ q they are a plain binary tree.
-template <typename T, int N, int U, int kOp, bool kTree>
+template <typename T, int N, int U, int kOp, bool kTree, bool kDstOnce>
 __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const FoldShared& sh, int nremote, unsigned v_lo,
                                              unsigned v_hi, int first, bool premul, T scalar) {
   using L = Lanes<T>;
@@ -261,7 +262,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 #pragma unroll
         for (int l = 0; l < V; ++l) out.e[l] = div_trunc(out.e[l], f.postdiv);
       }
-      fold_store<T>(dst, dst_aligned, sh, nremote, v, out, policy);
+      fold_store<T, kDstOnce>(dst, dst_aligned, sh, nremote, v, out, policy);
     }
   }
 }
@@ -281,7 +282,7 @@ __device__ __forceinline__ void fold_vectors(char* dst, bool dst_aligned, const 
 // tails, trees, recursive doubling over other counts. One B200, us a call: 7 ranks, 28 MB fp32 average, 677 by
 // that general path and 243 by vectors (111 CTAs); 9 ranks, 16 MiB e4m3, 748 and 165; 12 ranks, 16 MiB
 // fp32, 355 and 201.
-template <typename T, int kN>
+template <typename T, int kN, bool kDstOnce = true>
 static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, int nremote, size_t nbytes, size_t elem0,
                                              bool premul, T scalar) {
   const FoldSpec& f = sh.spec;
@@ -321,17 +322,17 @@ static __device__ __noinline__ void cta_fold(char* dst, const FoldShared& sh, in
     if constexpr (kN >= 2) {
       if (tree) {
         if (f.op == kSum)
-          fold_vectors<T, N, 1, kSum, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
+          fold_vectors<T, N, 1, kSum, true, kDstOnce>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
         else
-          fold_vectors<T, N, 1, -1, true>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
+          fold_vectors<T, N, 1, -1, true, kDstOnce>(dst, dst_aligned, sh, nremote, v, v_hi, 0, premul, scalar);
         v = v_hi;
         continue;
       }
     }
     if (f.op == kSum)
-      fold_vectors<T, N, U, kSum, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
+      fold_vectors<T, N, U, kSum, false, kDstOnce>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
     else
-      fold_vectors<T, N, 1, -1, false>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
+      fold_vectors<T, N, 1, -1, false, kDstOnce>(dst, dst_aligned, sh, nremote, v, v_hi, first, premul, scalar);
     v = v_hi;
   }
   for (unsigned e = nvec * V + t; e < total; e += nt) element(e);
