@@ -36,7 +36,7 @@ extern "C" {
  * device current it looks the array's device address up (cudaGetSymbolAddress) and clears the
  * array; make that first call before any stream capture begins. Later calls repeat the look-up
  * (so a device reset cannot leave a stale pointer behind). Every call ends with
- * cudaStreamSynchronize(stream).
+ * cudaStreamSynchronize(stream), so a stream that is being captured is refused before anything is enqueued.
  * Every call uses the same array and finds what the previous call left there: flags only grow
  * from call to call and the status words are cleared at the start of each call. Two calls that
  * overlap on the GPU (different streams, or different threads) therefore race on the array;

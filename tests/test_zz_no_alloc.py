@@ -88,3 +88,25 @@ def test_rejects_what_it_cannot_hold():
     assert b"HXCCL_NOALLOC_MAX_BYTES" in lib.hxcclNoAllocLastError()
     assert fn(5, _ptrs(x), _ptrs(x), 4, L.FLOAT32, L.SUM, None) == L.INVALID_ARGUMENT
     assert fn(2, _ptrs(x), _ptrs(x), 4, 99, L.SUM, None) == L.INVALID_ARGUMENT
+
+
+def test_a_capturing_stream_is_refused_at_the_door():
+    """Before the scratch is cleared: nothing of the call may end up in the graph."""
+    lib, fn = _entry()
+    x = [torch.full((1000,), float(r + 1), device="cuda") for r in range(2)]
+    y = [torch.zeros_like(t) for t in x]
+    marker = torch.zeros(1, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(torch.cuda.Stream()):
+        graph.capture_begin()
+        marker.fill_(1)
+        rc = fn(2, _ptrs(x), _ptrs(y), 1000, L.FLOAT32, L.SUM, torch.cuda.current_stream().cuda_stream)
+        text = lib.hxcclNoAllocLastError().decode()
+        graph.capture_end()
+    assert rc != 0 and "the stream is being captured" in text
+    graph.replay()
+    torch.cuda.synchronize()
+    assert float(marker) == 1 and not bool(y[0].any())
+    assert fn(2, _ptrs(x), _ptrs(y), 1000, L.FLOAT32, L.SUM, torch.cuda.current_stream().cuda_stream) == 0
+    assert all(bool((t == 3).all()) for t in y)
