@@ -13,8 +13,11 @@ __global__ void __launch_bounds__(512) k_xchg_copy(const __grid_constant__ XchgA
   __shared__ FoldShared sh;
   xchg_body<uint8_t, false>(a, blockIdx.x, gridDim.x, sh);
 }
-// Worlds run the copies, the lanes and the ring with two CTAs per SM (64 registers a thread suffice
-// there): 8 ranks, blocks of about 1 MiB at odd offsets: one CTA per SM 74 us, two 61 us.
+// Worlds run the copies, the lanes and the ring with two CTAs per SM, held to 64 registers a thread, at the
+// price of some spills. One B200, us a call, one CTA per SM and two: blocks of about 1 MiB at odd offsets on
+// 8 ranks 71 and 62, AllGather of 16 MiB blocks 700 and 611; ring, 2 ranks, 256 MiB fp32, 387 and 291; lanes,
+// ring shift of 32 MiB on 6 ranks 155 and 131, on 4 ranks 87 and 91, all pairs of 8 ranks, 4 MiB each, 184
+// and 161. AllGathers of a few MiB lose up to 10 % (2 ranks, 4 MiB blocks 13.4 and 14.8).
 __global__ void __launch_bounds__(512, 2) k_xchg_copy_world(const __grid_constant__ WorldArgs<XchgArgs> a) {
   __shared__ FoldShared sh;
   xchg_body<uint8_t, false>(a.rank[blockIdx.y], blockIdx.x, gridDim.x, sh);

@@ -13,7 +13,8 @@ namespace hx {
 // of the 32 KB a launch may carry). Staged through device memory they cost a stream
 // synchronisation (an earlier launch might still read the buffer) and a pageable copy per call:
 // 8 ranks, 41 KB bf16: 34.3 us a call staged, 22.6 us as parameters; 8 ranks, 8 B: 19.0 and 15.2 us.
-// Kernels made for up to kN ranks carry kN blocks only.
+// Kernels compiled for up to kN ranks carry kN blocks; the others (kN = 0: the copies, the ring, and the
+// folds' and lines' general forms) carry sixteen.
 template <typename Args, int kN = 0>
 struct WorldArgs {
   Args rank[kN ? kN : kMaxRanks];

@@ -160,11 +160,15 @@ __device__ __forceinline__ void st16_if(bool ok, void* p, uint4 v) {
                "r"(v.z), "r"(v.w), "l"(p), "r"(unsigned(ok))
                : "memory");
 }
-// Evict-first in the second-level cache, for data that is touched once: a caller's inputs and
+// Evict-first in the second-level cache, for data that is not read again soon: a caller's inputs and
 // outputs and, once read, the staged bytes. What is left to L2 are the bytes that a peer is still to
-// read. Staged traffic is two thirds of an AllReduce's, and most of it went to DRAM and back (ncu, 7
-// ranks, 28 MB fp32 average: 937 MB, L2 hit rate 13 %). One B200, us a call: 4 ranks, 16 MiB fp32 61.4 -> 56.9,
-// 8 ranks, 16 MiB e4m3 132.9 -> 128.8.
+// read. Staged traffic is two thirds of an AllReduce's, and much of it goes to DRAM and back. One B200, the
+// same build without the hints and with them, DRAM bytes of a launch (ncu) and us a call:
+//   4 ranks, 16 MiB fp32            216 and 177 MB, 62.8 and 59.0
+//   8 ranks, 16 MiB e4m3            659 and 504 MB, 136.2 and 131.6
+//   7 ranks, 28 MB fp32 average    1023 and 873 MB, 186.5 and 186.1
+//   8 ranks, AllGather of 1 MiB blocks              40.9 and 35.8
+// Messages of 1 to 4 MiB, which fit L2 as they are, lose 4 to 9 % (4 ranks, 4 MiB e4m3: 24.4 and 26.8).
 __device__ __forceinline__ unsigned long long once_policy() {
   unsigned long long p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
