@@ -104,7 +104,10 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
     v.half_off[0] = kHeaderBytes + p2p;
     v.half_off[1] = v.half_off[0] + half;
     v.half_bytes = half;
-    v.p2p_slot = kP2pSlotBytes / 2;  // 4 ranks, ring shift of 32 MiB: 100 us with 512 KiB slots, 95 with 256, 114 with 128
+    // One B200, us a call, 512 and 256 KiB slots: ring shift of 8 MiB on 2 ranks 32 and 30, on 8 ranks 60 and 52, of 64 MiB
+    // on 4 ranks 186 and 170, on 8 ranks 360 and 324. Where only two ranks move 32 MiB or more, 512 KiB is better
+    // (64 MiB: 131 and 150). 128 KiB: 4 ranks, 32 MiB, 114 against 95.
+    v.p2p_slot = kP2pSlotBytes / 2;
     v.wait_ns = uint64_t(wait_ms) * 1000000ull;
     v.rank = r;
     v.n = n;
@@ -119,8 +122,11 @@ hxcclResult_t hxcclWorldCreate(hxcclWorld_t* out, int n, int window_mb, int wait
   //   lines up to 64 KiB      2 ranks, 62 KiB: lines 10.6, one-shot 12.1; 8 ranks: 15.5 and 16.4. Rank counts whose
   //                           lines kernel is the general one only as long as every thread has one line:
   //                           7 ranks, e4m3, 42 KiB: 21.6 and 30.2, 46 KiB: 37.7 and 33.1; 12 ranks, 20 KiB: 19.2
-  //                           and 20.2, 28 KiB: 29.9 and 21.7
-  //   4 KiB grain             8 ranks, 512 KiB two-shot: 17.2, with 16 KiB 22.4; 1 MiB 19.3 and 23.1
+  //                           and 20.2, 28 KiB: 29.9 and 21.7 (on 7 ranks lines win again near 60 KiB of a
+  //                           narrow type, 37.4 and 40.3 in e4m3, and lose in fp32, 19.1 and 17.5)
+  //   4 KiB grain             with 16 KiB: 12 ranks, 512 KiB 32.7 against 20.3; 8 ranks 20.8 and 16.7; 6 ranks 23.3 and
+  //                           18.2; 2 ranks, 1 MiB e4m3 20.4 and 18.7. Some sizes lose (4 ranks, 256 KiB e4m3
+  //                           13.8 against 16.2)
   //   ring from 40 MiB on two ranks (32 MiB: ring 53, two-shot 50; 40 MiB: 71 and 95), from 56 MiB on more, for 4-, 2-
   //                           and 1-byte types (4 ranks, 48 MiB: 189 and 171; 56 MiB: 194 and 200; 8 ranks:
   //                           400 and 381, 409 and 440; 12 ranks: 623 and 606, 646 and 703). Where the last
